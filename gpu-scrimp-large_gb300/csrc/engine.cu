@@ -456,6 +456,14 @@ SeriesDev to_dev(const SeriesBufs& s, int64_t n, int64_t ns) {
   return d;
 }
 
+// Window statistics of one series (`raw`, n samples) into its buffers.
+void launch_stats(const double* raw, int64_t n, int64_t m, bool ultra, const SeriesBufs& s,
+                  cudaStream_t st) {
+  const StatsJob j{raw, n, m, s.bshift, s.T, s.mean, s.inv, s.df, s.dg,
+                   s.T32, s.bhi, s.blo, s.mu_rel, s.inv32, s.df32, s.dg32};
+  stats_kernel<<<static_cast<unsigned>(stats_blocks(n - m + 1)), kStatsThreads, 0, st>>>(j, ultra ? 1 : 0);
+}
+
 // One problem's chunk of tensor-core anchors: anchor rows s0 .. s0 + nrows
 // - 1 of the row series against every diagonal of the problem, into `table`
 // (nrows x wp_pad floats, the layout of anchor_tc.cu).
@@ -529,10 +537,7 @@ int tc_self_check(Workspace& ws, cudaStream_t st, std::string* msg, bool wait_te
   SeriesBufs sb{};
   sb.bshift = block_shift(m);
   if ((rc = alloc_series(ws, 0, n, ns, &sb, msg))) return rc;
-  const int chunk = 64;
-  stats_kernel<<<static_cast<unsigned>(((ns + chunk - 1) / chunk + 127) / 128), 128, 0, st>>>(
-      raw, n, m, 0, chunk, sb.bshift, sb.T, sb.T32, sb.bhi, sb.blo, sb.mu_rel, sb.mean, sb.inv,
-      sb.df, sb.dg, sb.inv32, sb.df32, sb.dg32);
+  launch_stats(raw, n, m, false, sb, st);
   CUDA_TRY(cudaGetLastError());
   Problem pr{};
   pr.R = pr.C = to_dev(sb, n, ns);
@@ -751,20 +756,11 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   SeriesBufs sa{}, sb{};
   sa.bshift = sb.bshift = block_shift(m);
   if ((rc = alloc_series(ws, 0, na, plan.ns_a, &sa, msg))) return rc;
-  const int chunk = 64;
-  {
-    const int64_t threads = (plan.ns_a + chunk - 1) / chunk;
-    stats_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(
-        dA, na, m, ultra ? 1 : 0, chunk, sa.bshift, sa.T, sa.T32, sa.bhi, sa.blo, sa.mu_rel,
-        sa.mean, sa.inv, sa.df, sa.dg, sa.inv32, sa.df32, sa.dg32);
-    launches += 1;
-  }
+  launch_stats(dA, na, m, ultra, sa, st);
+  launches += 1;
   if (a->has_b) {
     if ((rc = alloc_series(ws, 1, nb, plan.ns_b, &sb, msg))) return rc;
-    const int64_t threads = (plan.ns_b + chunk - 1) / chunk;
-    stats_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(
-        dB, nb, m, ultra ? 1 : 0, chunk, sb.bshift, sb.T, sb.T32, sb.bhi, sb.blo, sb.mu_rel,
-        sb.mean, sb.inv, sb.df, sb.dg, sb.inv32, sb.df32, sb.dg32);
+    launch_stats(dB, nb, m, ultra, sb, st);
     launches += 1;
   } else {
     sb = sa;
@@ -1401,11 +1397,7 @@ int window_stats(Workspace& ws, const double* series, int64_t n, int64_t m, int 
   SeriesBufs sb{};
   sb.bshift = block_shift(m);
   if ((rc = alloc_series(ws, 0, n, ns, &sb, msg))) return rc;
-  const int chunk = 64;
-  const int64_t threads = (ns + chunk - 1) / chunk;
-  stats_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(
-      raw, n, m, ultra, chunk, sb.bshift, sb.T, sb.T32, sb.bhi, sb.blo, sb.mu_rel, sb.mean,
-      sb.inv, sb.df, sb.dg, sb.inv32, sb.df32, sb.dg32);
+  launch_stats(raw, n, m, ultra != 0, sb, st);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaMemcpyAsync(mean, sb.mean, ns * 8, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaMemcpyAsync(invnorm, sb.inv, ns * 8, cudaMemcpyDeviceToHost, st));
@@ -1756,21 +1748,12 @@ int run_device_noalloc(const NoAllocDevice& dv, const scamp_c_args* a, scamp_c_r
   const SeriesBufs sb_carved = sb;
 
   uint32_t launches = 0;
-  const int chunk = 64;
   const double* dA = a->timeseries_a;
   const double* dB = a->has_b ? a->timeseries_b : a->timeseries_a;
-  {
-    const int64_t threads = (plan.ns_a + chunk - 1) / chunk;
-    stats_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(
-        dA, na, m, ultra ? 1 : 0, chunk, sa.bshift, sa.T, sa.T32, sa.bhi, sa.blo, sa.mu_rel,
-        sa.mean, sa.inv, sa.df, sa.dg, sa.inv32, sa.df32, sa.dg32);
-    ++launches;
-  }
+  launch_stats(dA, na, m, ultra, sa, st);
+  ++launches;
   if (a->has_b) {
-    const int64_t threads = (plan.ns_b + chunk - 1) / chunk;
-    stats_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, st>>>(
-        dB, nb, m, ultra ? 1 : 0, chunk, sb.bshift, sb.T, sb.T32, sb.bhi, sb.blo, sb.mu_rel,
-        sb.mean, sb.inv, sb.df, sb.dg, sb.inv32, sb.df32, sb.dg32);
+    launch_stats(dB, nb, m, ultra, sb, st);
     ++launches;
   } else {
     sb = sa;
@@ -2210,14 +2193,12 @@ int run_batch(Workspace& ws, const scamp_c_args* args, scamp_c_result* res, int 
     std::memcpy(h_raw + ser[k].off_n, args[k].timeseries_a, ser[k].n * 8);
     std::memcpy(h_prof + ser[k].off_ns, res[k].profile_a, ser[k].ns * 8);
   }
-  const int chunk = 64;
   std::vector<StatsJob> jobs(count);
   std::vector<int64_t> jpre(count + 1, 0);
   for (int k = 0; k < count; ++k) {
     const BatchSeries& b = ser[k];
     jobs[k] = batch_stats_job(A1, b.off_n, b.off_ns, b.off_blk, b.bshift, b.n, b.m);
-    const int64_t threads = (b.ns + chunk - 1) / chunk;
-    jpre[k + 1] = jpre[k] + (threads + 127) / 128;
+    jpre[k + 1] = jpre[k] + stats_blocks(b.ns);
   }
   const KeyLayout kl = make_key_layout(ns_max);
   const int W = mixed_1nn_band_width();
@@ -2249,7 +2230,7 @@ int run_batch(Workspace& ws, const scamp_c_args* args, scamp_c_result* res, int 
     paa_jobs.push_back(PaaJob{d_raw + b.off_n, A2.raw + b.off_n2, b.n2, b.f});
     paapre.push_back(paapre.back() + b.n2);
     jobs2.push_back(batch_stats_job(A2, b.off_n2, b.off_ns2, b.off_blk2, b.bshift2, b.n2, b.m2));
-    jpre2.push_back(jpre2.back() + ((b.ns2 + chunk - 1) / chunk + 127) / 128);
+    jpre2.push_back(jpre2.back() + stats_blocks(b.ns2));
     const SeriesDev sd2 = batch_series_dev(A2, b.off_n2, b.off_ns2, b.off_blk2, b.bshift2, b.n2, b.ns2);
     const Problem pr2 = batch_problem(sd2, A2.keys + b.off_ns2, b.excl2, b.m2, b.K2, band_total2, W,
                                       &bpre2);
@@ -2384,16 +2365,16 @@ int run_batch(Workspace& ws, const scamp_c_args* args, scamp_c_result* res, int 
   if (!ws.batch_exec || ws.batch_key != key) {
     auto enqueue = [&]() -> cudaError_t {
       cudaError_t e;
-      stats_batch_kernel<<<static_cast<unsigned>(jpre[count]), 128, 0, st>>>(d_jobs, d_jpre, count, 0,
-                                                                              chunk);
+      stats_batch_kernel<<<static_cast<unsigned>(jpre[count]), kStatsThreads, 0, st>>>(d_jobs, d_jpre,
+                                                                                        count);
       profile_to_keys_kernel<<<static_cast<unsigned>((Nns + 255) / 256), 256, 0, st>>>(d_prof, d_keys,
                                                                                        Nns, kl);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       if (seeded) {
         const int nj = static_cast<int>(nseed_jobs);
         paa_batch_kernel<<<static_cast<unsigned>(paa_blocks), 256, 0, st>>>(d_paa, d_paapre, nj);
-        stats_batch_kernel<<<static_cast<unsigned>(jpre2.back()), 128, 0, st>>>(d_jobs2, d_jpre2, nj, 0,
-                                                                                 chunk);
+        stats_batch_kernel<<<static_cast<unsigned>(jpre2.back()), kStatsThreads, 0, st>>>(d_jobs2,
+                                                                                           d_jpre2, nj);
         fill_key_floor_kernel<<<static_cast<unsigned>(fill2_blocks), 256, 0, st>>>(A2.keys, N2ns,
                                                                                     kSeedFloor, kl);
         diag_seed_kernel<<<static_cast<unsigned>(seed2_blocks), 256, 0, st>>>(d_probs2, d_wpre2, nj, kl);

@@ -243,20 +243,17 @@ struct StatsJob {
   double *T_clean, *mean, *inv, *df, *dg;
   float *T32, *bhi, *blo, *mu_rel, *inv32, *df32, *dg32;
 };
+// Statistics launches: one warp per kStatsChunk windows of a series.
+constexpr int kStatsChunk = 64;
+constexpr int kStatsThreads = 128;
+inline int64_t stats_blocks(int64_t ns) {
+  constexpr int64_t per_block = kStatsChunk * (kStatsThreads / 32);
+  return (ns + per_block - 1) / per_block;
+}
+__global__ void stats_kernel(StatsJob j, int ultra);
 // Block b of the launch works for job j with block_prefix[j] <= b < block_prefix[j + 1].
 __global__ void stats_batch_kernel(const StatsJob* __restrict__ jobs,
-                                   const int64_t* __restrict__ block_prefix, int njobs,
-                                   int ultra, int chunk);
-
-__global__ void stats_kernel(const double* __restrict__ T_raw, int64_t n,
-                             int64_t m, int ultra, int chunk, int bshift,
-                             double* __restrict__ T_clean, float* __restrict__ T32,
-                             float* __restrict__ bhi, float* __restrict__ blo,
-                             float* __restrict__ mu_rel,
-                             double* __restrict__ mean, double* __restrict__ inv,
-                             double* __restrict__ df, double* __restrict__ dg,
-                             float* __restrict__ inv32, float* __restrict__ df32,
-                             float* __restrict__ dg32);
+                                   const int64_t* __restrict__ block_prefix, int njobs);
 
 // ULTRA update terms of one series: role_b 0 gives the "A" terms, 1 the "B"
 // terms (stats.cu); T is the cleaned series, mean its window means.

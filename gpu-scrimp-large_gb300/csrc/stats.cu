@@ -2,11 +2,12 @@
 //
 // Replaces the reference's host-side, sequential precompute
 // (src/cpu_stats.cpp:11-160, called from src/SCAMP.cpp:195-206) with one
-// kernel.  Each thread owns `chunk` consecutive windows: it sums its first
-// window directly, then slides (the reference's rolling, TwoSum-compensated
-// update), so the rounding error restarts every `chunk` windows instead of
-// growing over the whole series.  ULTRA precision sums every window directly
-// (the reference's brute-force O(nm) option, src/cpu_stats.cpp:31-41, 85-97).
+// kernel.  Each warp owns kStatsChunk consecutive windows: it sums its first
+// window directly, then the others from it (the reference's rolling,
+// TwoSum-compensated update, as scans over the warp's lanes), so the rounding
+// error restarts every kStatsChunk windows instead of growing over the whole
+// series.  ULTRA precision sums every window directly (the reference's
+// brute-force O(nm) option, src/cpu_stats.cpp:31-41, 85-97).
 //
 // Semantics kept exactly:
 //  - non-finite samples become 0 and poison every window holding them
@@ -39,166 +40,236 @@ __device__ __forceinline__ void acc2(double& s, double& c, double x) {
 
 }  // namespace
 
-// Statistics of windows [tid * chunk, (tid + 1) * chunk) of one series.
-__device__ __forceinline__ void stats_body(int64_t tid, const double* __restrict__ T_raw, int64_t n,
-                             int64_t m, int ultra, int chunk, int bshift,
-                             double* __restrict__ T_clean, float* __restrict__ T32,
-                             float* __restrict__ bhi, float* __restrict__ blo,
-                             float* __restrict__ mu_rel,
-                             double* __restrict__ mean, double* __restrict__ inv,
-                             double* __restrict__ df, double* __restrict__ dg,
-                             float* __restrict__ inv32, float* __restrict__ df32,
-                             float* __restrict__ dg32) {
+// Sum of two compensated sums: (s, c) += (s2, c2).
+__device__ __forceinline__ void add2(double& s, double& c, double s2, double c2) {
+  acc2(s, c, s2);
+  c += c2;
+}
+
+// One window's outputs from its mean (mu + mu_lo), the next window's mean
+// and its sum of squared deviations.
+struct StatsOut {
+  double *mean, *inv, *df, *dg;
+  float *mu_rel, *inv32, *df32, *dg32;
+};
+__device__ __forceinline__ void write_window(const StatsOut& o, int64_t w, double x_out, double x_in,
+                                             bool has_next, double mu, double mu_lo, double mu_next,
+                                             double mu_next_lo, double ssd, bool nan_window,
+                                             double block_off) {
+  const double iv = (nan_window || !(ssd > kFlatnessEpsilon)) ? nan("") : 1.0 / sqrt(ssd);
+  double f = 0, g = 0;
+  if (has_next) {
+    f = (x_in - x_out) / 2.0;
+    g = ((x_in - mu_next) - mu_next_lo) + ((x_out - mu) - mu_lo);
+  }
+  o.mean[w] = mu;
+  o.mu_rel[w] = static_cast<float>((mu - block_off) + mu_lo);
+  o.inv[w] = iv;
+  o.df[w] = f;
+  o.dg[w] = g;
+  o.inv32[w] = static_cast<float>(iv);
+  o.df32[w] = static_cast<float>(f);
+  o.dg32[w] = static_cast<float>(g);
+}
+
+// Statistics of windows [chunk * kStatsChunk, (chunk + 1) * kStatsChunk) of
+// one series, by one warp (every lane calls it; `lane` its lane).
+//
+// The lanes share the direct sums of the chunk's first window (each sums
+// every 32nd sample, compensated; the partial sums meet in a shuffle tree).
+// Window w's sum is the first window's plus the differences x[v + m] - x[v],
+// v < w, and its sum of squares the first window's plus the reference's
+// recurrence terms (src/cpu_stats.cpp:114-117): both are compensated scans
+// over the lanes, 32 windows at a time.  Per window that leaves one
+// divide and one square root per lane and no chain from window to window.
+// Bound by the FP64 pipe: 2 m x 8 additions per 64 windows plus about 100
+// per window.  One thread per 64-window chunk, which this replaces, was bound by
+// its own chain of FP64 latencies at every size: 276 / 348 / 1158 us at 1000
+// (m = 50) / 131072 (m = 100) / 40009 samples (m = 1024).
+__device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double* __restrict__ T_raw,
+                                           int64_t n, int64_t m, int ultra, int bshift,
+                                           double* __restrict__ T_clean, float* __restrict__ T32,
+                                           float* __restrict__ bhi, float* __restrict__ blo,
+                                           const StatsOut& o) {
+  constexpr unsigned kAll = 0xffffffffu;
   const int64_t ns = n - m + 1;
-  const int64_t w0 = tid * chunk;
+  const int64_t w0 = chunk * kStatsChunk;
   if (w0 >= ns) return;
-  const int64_t w1 = (w0 + chunk < ns) ? w0 + chunk : ns;
+  const int64_t w1 = (w0 + kStatsChunk < ns) ? w0 + kStatsChunk : ns;
 
   // Cleaned samples owned by this chunk (the last chunk also owns the tail).
   // Block offsets are the blocks' first (cleaned) samples.
   auto block_off = [&](int64_t b) { return clean(T_raw[b << bshift]); };
   {
     const int64_t s_end = (w1 == ns) ? n : w1;
-    for (int64_t t = w0; t < s_end; ++t) {
+    for (int64_t t = w0 + lane; t < s_end; t += 32) {
       const double c = clean(T_raw[t]);
       T_clean[t] = c;
       const int64_t b = t >> bshift;
-      const double o = block_off(b);
-      T32[t] = static_cast<float>(c - o);
+      const double off = block_off(b);
+      T32[t] = static_cast<float>(c - off);
       if ((b << bshift) == t) {
-        const float hi = static_cast<float>(o);
+        const float hi = static_cast<float>(off);
         bhi[b] = hi;
-        blo[b] = static_cast<float>(o - static_cast<double>(hi));
+        blo[b] = static_cast<float>(off - static_cast<double>(hi));
       }
     }
   }
 
-  // Mean and NaN status of window w0, and the position of the last
-  // non-finite sample seen so far.
-  int64_t last_bad = -1;
-  double ps = 0, pc = 0;
-  for (int64_t t = 0; t < m; ++t) {
-    const double x = T_raw[w0 + t];
-    if (!isfinite(x)) last_bad = w0 + t;
-    acc2(ps, pc, clean(x));
-  }
   // The mean is carried as mu + mu_lo: the low part restores the digits the
   // division drops, which matters for series with a large offset relative
   // to their variation (dg subtracts the mean from the raw samples).
   const double md = static_cast<double>(m);
-  double mu = (ps + pc) / md;
-  double mu_lo = (fma(-mu, md, ps) + pc) / md;
+  auto mean_of = [&](double ps, double pc, double& mu, double& mu_lo) {
+    mu = (ps + pc) / md;
+    mu_lo = (fma(-mu, md, ps) + pc) / md;
+  };
 
-  // ssd of window w0, direct.
-  double ss = 0, sc = 0;
-  for (int64_t t = 0; t < m; ++t) {
-    const double v = clean(T_raw[w0 + t]) - mu;
-    acc2(ss, sc, v * v);
-  }
-
-  for (int64_t w = w0; w < w1; ++w) {
-    // Mean of window w+1 (needed by dg[w]).
-    double mu_next = 0, mu_next_lo = 0;
-    int64_t last_bad_next = last_bad;
-    const bool has_next = (w + 1 < ns);
-    double ps_n = ps, pc_n = pc;
-    if (has_next) {
-      const double x_out = clean(T_raw[w]);
-      const double x_in_raw = T_raw[w + m];
-      if (!isfinite(x_in_raw)) last_bad_next = w + m;
-      const double x_in = clean(x_in_raw);
-      if (ultra) {
+  if (ultra) {
+    // every window summed directly, in order, by its own lane
+    for (int64_t w = w0 + lane; w < w1; w += 32) {
+      double ps = 0, pc = 0;
+      bool bad = false;
+      for (int64_t t = 0; t < m; ++t) {
+        const double x = T_raw[w + t];
+        bad = bad || !isfinite(x);
+        acc2(ps, pc, clean(x));
+      }
+      double mu, mu_lo, mu_next = 0, mu_next_lo = 0;
+      mean_of(ps, pc, mu, mu_lo);
+      double ss = 0, sc = 0;
+      for (int64_t t = 0; t < m; ++t) {
+        const double v = clean(T_raw[w + t]) - mu;
+        acc2(ss, sc, v * v);
+      }
+      const bool has_next = w + 1 < ns;
+      if (has_next) {
         double s2 = 0, c2 = 0;
         for (int64_t t = 0; t < m; ++t) acc2(s2, c2, clean(T_raw[w + 1 + t]));
-        ps_n = s2;
-        pc_n = c2;
-      } else {
-        acc2(ps_n, pc_n, -x_out);
-        acc2(ps_n, pc_n, x_in);
+        mean_of(s2, c2, mu_next, mu_next_lo);
       }
-      mu_next = (ps_n + pc_n) / md;
-      mu_next_lo = (fma(-mu_next, md, ps_n) + pc_n) / md;
+      write_window(o, w, clean(T_raw[w]), has_next ? clean(T_raw[w + m]) : 0.0, has_next, mu, mu_lo,
+                   mu_next, mu_next_lo, ss + sc, bad, block_off(w >> bshift));
     }
+    return;
+  }
 
-    // Window w statistics.  A near-flat ssd from the recurrence is summed
-    // again directly, so the flatness rule sees no accumulated residue.
-    double ssd = ss + sc;
-    if (ssd <= 1e3 * kFlatnessEpsilon && !ultra) {
-      double s2 = 0, c2 = 0;
-      for (int64_t t = 0; t < m; ++t) {
-        const double v = (clean(T_raw[w + t]) - mu) - mu_lo;
-        acc2(s2, c2, v * v);
-      }
-      ssd = s2 + c2;
-    }
-    const bool nan_window = last_bad >= w;  // a non-finite sample in [w, w+m)
-    double iv;
-    if (nan_window || !(ssd > kFlatnessEpsilon)) {
-      iv = nan("");
-    } else {
-      iv = 1.0 / sqrt(ssd);
-    }
-    double f = 0, g = 0;
-    if (has_next) {
-      const double a = clean(T_raw[w]);
-      const double b = clean(T_raw[w + m]);
-      f = (b - a) / 2.0;
-      g = ((b - mu_next) - mu_next_lo) + ((a - mu) - mu_lo);
-    }
-    mean[w] = mu;
-    mu_rel[w] = static_cast<float>((mu - block_off(w >> bshift)) + mu_lo);
-    inv[w] = iv;
-    df[w] = f;
-    dg[w] = g;
-    inv32[w] = static_cast<float>(iv);
-    df32[w] = static_cast<float>(f);
-    dg32[w] = static_cast<float>(g);
+  // Window w0: sum, mean, sum of squared deviations, last non-finite sample.
+  double ps = 0, pc = 0;
+  int64_t last_bad = -1;
+  for (int64_t t = lane; t < m; t += 32) {
+    const double x = T_raw[w0 + t];
+    if (!isfinite(x)) last_bad = w0 + t;
+    acc2(ps, pc, clean(x));
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    add2(ps, pc, __shfl_xor_sync(kAll, ps, s), __shfl_xor_sync(kAll, pc, s));
+    const int64_t ob = __shfl_xor_sync(kAll, last_bad, s);
+    last_bad = ob > last_bad ? ob : last_bad;
+  }
+  // (the tree adds in an order that depends on the lane: one lane's result)
+  ps = __shfl_sync(kAll, ps, 0);
+  pc = __shfl_sync(kAll, pc, 0);
+  double mu0, mu0_lo;
+  mean_of(ps, pc, mu0, mu0_lo);
+  double ss = 0, sc = 0;
+  for (int64_t t = lane; t < m; t += 32) {
+    const double v = clean(T_raw[w0 + t]) - mu0;
+    acc2(ss, sc, v * v);
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    add2(ss, sc, __shfl_xor_sync(kAll, ss, s), __shfl_xor_sync(kAll, sc, s));
+  ss = __shfl_sync(kAll, ss, 0);
+  sc = __shfl_sync(kAll, sc, 0);
 
-    if (!has_next) break;
-    // Advance ssd to window w+1: the reference's recurrence
-    // (src/cpu_stats.cpp:114-117), accumulated with compensation; ULTRA
-    // recomputes it directly.
-    if (ultra) {
-      double s2 = 0, c2 = 0;
-      for (int64_t t = 0; t < m; ++t) {
-        const double v = clean(T_raw[w + 1 + t]) - mu_next;
-        acc2(s2, c2, v * v);
-      }
-      ss = s2;
-      sc = c2;
-    } else {
-      // With the means' low parts, so that a large offset's rounded mean
-      // does not leave a per-step residue (b - a)(delta_w + delta_w+1).
-      const double a = clean(T_raw[w]);
-      const double b = clean(T_raw[w + m]);
-      acc2(ss, sc, (((a - mu) - mu_lo) + ((b - mu_next) - mu_next_lo)) * (b - a));
+  // 32 windows at a time; (ps, pc) and (ss, sc) are those of window wb.
+  for (int64_t wb = w0; wb < w1; wb += 32) {
+    const int64_t w = wb + lane;
+    const bool active = w < w1;
+    const bool has_next = w + 1 < ns;
+    const double x_out = active ? clean(T_raw[w]) : 0.0;
+    const double x_raw = (active && has_next) ? T_raw[w + m] : 0.0;
+    const double x_in = clean(x_raw);
+    // sums of windows wb + 1 .. wb + 32: inclusive scan of the differences
+    double ds = 0, dc = 0;
+    acc2(ds, dc, x_in);
+    acc2(ds, dc, -x_out);
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const double us = __shfl_up_sync(kAll, ds, s), uc = __shfl_up_sync(kAll, dc, s);
+      if (lane >= s) add2(ds, dc, us, uc);
     }
-    ps = ps_n;
-    pc = pc_n;
-    mu = mu_next;
-    mu_lo = mu_next_lo;
-    last_bad = last_bad_next;
+    double ns_s = ps, ns_c = pc;  // the sum of window w + 1
+    add2(ns_s, ns_c, ds, dc);
+    double mu_next, mu_next_lo;
+    mean_of(ns_s, ns_c, mu_next, mu_next_lo);
+    double mu = __shfl_up_sync(kAll, mu_next, 1), mu_lo = __shfl_up_sync(kAll, mu_next_lo, 1);
+    if (lane == 0) {
+      mu = mu0;
+      mu_lo = mu0_lo;
+    }
+    // Sums of squares: the recurrence's terms with the means' low parts, so
+    // that a large offset's rounded mean does not leave a per-step residue
+    // (b - a)(delta_w + delta_w+1).
+    double es = 0, ec = 0;
+    if (active && has_next)
+      es = (((x_out - mu) - mu_lo) + ((x_in - mu_next) - mu_next_lo)) * (x_in - x_out);
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const double us = __shfl_up_sync(kAll, es, s), uc = __shfl_up_sync(kAll, ec, s);
+      if (lane >= s) add2(es, ec, us, uc);
+    }
+    double nss = ss, nsc = sc;  // of window w + 1
+    add2(nss, nsc, es, ec);
+    double ssd_s = __shfl_up_sync(kAll, nss, 1), ssd_c = __shfl_up_sync(kAll, nsc, 1);
+    if (lane == 0) {
+      ssd_s = ss;
+      ssd_c = sc;
+    }
+    // the last non-finite sample of window w: one in front of sample w + m,
+    // or the chunk's running one
+    const unsigned bad = __ballot_sync(kAll, active && has_next && !isfinite(x_raw));
+    const unsigned before = bad & ((1u << lane) - 1u);
+    int64_t lb = last_bad;
+    if (before) lb = wb + m + (31 - __clz(before));
+    if (active) {
+      // A near-flat ssd from the recurrence is summed again directly, so the
+      // flatness rule sees no accumulated residue.
+      double ssd = ssd_s + ssd_c;
+      if (ssd <= 1e3 * kFlatnessEpsilon) {
+        double s2 = 0, c2 = 0;
+        for (int64_t t = 0; t < m; ++t) {
+          const double v = (clean(T_raw[w + t]) - mu) - mu_lo;
+          acc2(s2, c2, v * v);
+        }
+        ssd = s2 + c2;
+      }
+      write_window(o, w, x_out, x_in, has_next, mu, mu_lo, mu_next, mu_next_lo, ssd, lb >= w,
+                   block_off(w >> bshift));
+    }
+    // window wb + 32
+    ps = __shfl_sync(kAll, ns_s, 31);
+    pc = __shfl_sync(kAll, ns_c, 31);
+    ss = __shfl_sync(kAll, nss, 31);
+    sc = __shfl_sync(kAll, nsc, 31);
+    mu0 = __shfl_sync(kAll, mu_next, 31);
+    mu0_lo = __shfl_sync(kAll, mu_next_lo, 31);
+    if (bad) last_bad = wb + m + (31 - __clz(bad));
   }
 }
 
-
-__global__ void stats_kernel(const double* __restrict__ T_raw, int64_t n,
-                             int64_t m, int ultra, int chunk, int bshift,
-                             double* __restrict__ T_clean, float* __restrict__ T32,
-                             float* __restrict__ bhi, float* __restrict__ blo,
-                             float* __restrict__ mu_rel,
-                             double* __restrict__ mean, double* __restrict__ inv,
-                             double* __restrict__ df, double* __restrict__ dg,
-                             float* __restrict__ inv32, float* __restrict__ df32,
-                             float* __restrict__ dg32) {
-  const int64_t tid = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  stats_body(tid, T_raw, n, m, ultra, chunk, bshift, T_clean, T32, bhi, blo, mu_rel, mean, inv,
-             df, dg, inv32, df32, dg32);
+__global__ void __launch_bounds__(kStatsThreads) stats_kernel(StatsJob j, int ultra) {
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * kStatsThreads + threadIdx.x) >> 5;
+  const StatsOut o{j.mean, j.inv, j.df, j.dg, j.mu_rel, j.inv32, j.df32, j.dg32};
+  stats_body(warp, threadIdx.x & 31, j.T_raw, j.n, j.m, ultra, j.bshift, j.T_clean, j.T32, j.bhi,
+             j.blo, o);
 }
 
-__global__ void stats_batch_kernel(const StatsJob* __restrict__ jobs,
-                                   const int64_t* __restrict__ block_prefix, int njobs,
-                                   int ultra, int chunk) {
+__global__ void __launch_bounds__(kStatsThreads)
+stats_batch_kernel(const StatsJob* __restrict__ jobs, const int64_t* __restrict__ block_prefix,
+                   int njobs) {
   const int64_t b = blockIdx.x;
   int lo = 0, hi = njobs;
   while (hi - lo > 1) {
@@ -206,9 +277,10 @@ __global__ void stats_batch_kernel(const StatsJob* __restrict__ jobs,
     if (block_prefix[mid] <= b) lo = mid; else hi = mid;
   }
   const StatsJob& j = jobs[lo];
-  const int64_t tid = (b - block_prefix[lo]) * blockDim.x + threadIdx.x;
-  stats_body(tid, j.T_raw, j.n, j.m, ultra, chunk, j.bshift, j.T_clean, j.T32, j.bhi, j.blo,
-             j.mu_rel, j.mean, j.inv, j.df, j.dg, j.inv32, j.df32, j.dg32);
+  const int64_t warp = ((b - block_prefix[lo]) * kStatsThreads + threadIdx.x) >> 5;
+  const StatsOut o{j.mean, j.inv, j.df, j.dg, j.mu_rel, j.inv32, j.df32, j.dg32};
+  stats_body(warp, threadIdx.x & 31, j.T_raw, j.n, j.m, 0, j.bshift, j.T_clean, j.T32, j.bhi, j.blo,
+             o);
 }
 
 // ULTRA's update terms (the reference's compute_combined_stats_cpu,
