@@ -125,6 +125,25 @@ int64_t cold_anchor_interval(int64_t m) {
   return std::min<int64_t>(std::max<int64_t>(4096, 2 * m), std::max<int64_t>(1024, 8 * m));
 }
 
+// The exact form serves FP64 1NN joins of at least this many cells: smaller
+// ones spend their time raising bests from nothing, every step flagged
+// (whole join, FP64 band kernel against exact form: 6001 samples, m = 33,
+// 0.33 / 0.68 ms; 15000 samples, m = 64, 1.64 / 0.73 ms).
+constexpr uint64_t kExactMinCells = uint64_t{1} << 25;
+// Its longest window: the FP32 bounds are first order in m 2^-24, and the
+// rounding of their own sums is covered up to here.
+constexpr int64_t kExactMaxWindow = 65536;
+
+// Verification requests a unit of the exact form may make before the FP64
+// band kernel takes it: one for every fourth cell.  A request costs the FP64
+// pipe 3 m operations against 4 for a cell of the FP64 kernel, but most are
+// ruled out by the final bests before that: joins that start cold make up to
+// a hundred per window (30000 samples, m = 1024: 3.2 ms with this budget,
+// 7.4 ms with one request per 12 cells).
+unsigned exact_request_budget(int64_t K, int W) {
+  return static_cast<unsigned>(2 * K * W / 4);
+}
+
 // Rows between seeds of the FP64 form.  The FP64 recurrence drifts by
 // ~2^-53 per row, so seeds only bound the work lost to them: 32 m rows keep
 // the direct-dot seeds at 1/32 of the FP64 pipe's work.
@@ -313,6 +332,7 @@ struct Workspace {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t evk0 = nullptr, evk1 = nullptr;  // around the join kernels
   cudaEvent_t evkv = nullptr;                   // before the verification kernel
+  int fp64_occ = 1;                             // resident join_fp64_kernel CTAs per SM
   bool timed_kernel = false;
   bool timed_verify = false;
   // the mixed form's largest trusted drift margin (work counter 4) is the
@@ -392,7 +412,7 @@ enum Slot {
   S_PREFIX, S_COUNTER, S_T32_A, S_T32_B, S_BHI_A, S_BLO_A, S_MUREL_A,
   S_BHI_B, S_BLO_B, S_MUREL_B, S_VREQ, S_PAA_A, S_PAA_B, S_SEED_A, S_SEED_B,
   S_BATCH, S_MAX_A, S_MAX_B, S_KNN_A, S_KNN_B, S_MAT,
-  S_TC_TAB, S_TC_W, S_TC_XS, S_TC_RAW, S_TC_OUT, S_TC_XI,
+  S_TC_TAB, S_TC_W, S_TC_XS, S_TC_RAW, S_TC_OUT, S_TC_XI, S_FP64_LIST,
 };
 
 #define CUDA_TRY(expr)                                                     \
@@ -458,9 +478,9 @@ SeriesDev to_dev(const SeriesBufs& s, int64_t n, int64_t ns) {
 
 // Window statistics of one series (`raw`, n samples) into its buffers.
 void launch_stats(const double* raw, int64_t n, int64_t m, bool ultra, const SeriesBufs& s,
-                  cudaStream_t st) {
+                  cudaStream_t st, unsigned* range = nullptr) {
   const StatsJob j{raw, n, m, s.bshift, s.T, s.mean, s.inv, s.df, s.dg,
-                   s.T32, s.bhi, s.blo, s.mu_rel, s.inv32, s.df32, s.dg32};
+                   s.T32, s.bhi, s.blo, s.mu_rel, s.inv32, s.df32, s.dg32, range};
   stats_kernel<<<static_cast<unsigned>(stats_blocks(n - m + 1)), kStatsThreads, 0, st>>>(j, ultra ? 1 : 0);
 }
 
@@ -741,11 +761,16 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
     CUDA_TRY(cudaEventRecord(ws.ev0, st));
   }
 
+  // FP64 1NN joins on the mixed band kernel: cells that deterministic bounds
+  // cannot rule out get their FP64 r, so the profile is the FP64 one
+  const bool exact = is_1nn && a->precision_type == SCAMP_PRECISION_DOUBLE && !nested &&
+                     plan.cells >= kExactMinCells && m <= kExactMaxWindow;
+
   // ---- seeds: block-averaged pre-pass (mixed 1NN joins that pay for it) ----
   NvtxRange nvtx_join(nested ? "seeding pre-pass join" : "join");
   uint64_t *seed_a = nullptr, *seed_b = nullptr;
   int64_t seed_ns_a = 0, seed_ns_b = 0;
-  if (!nested && mixed && is_1nn && seedable(a, plan)) {
+  if (!nested && (mixed || exact) && is_1nn && seedable(a, plan)) {
     if ((rc = seed_prepass(ws, a, plan, dA, dB, st, &seed_a, &seed_b, &seed_ns_a, &seed_ns_b,
                            &launches, msg)))
       return rc;
@@ -756,11 +781,19 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   SeriesBufs sa{}, sb{};
   sa.bshift = sb.bshift = block_shift(m);
   if ((rc = alloc_series(ws, 0, na, plan.ns_a, &sa, msg))) return rc;
-  launch_stats(dA, na, m, ultra, sa, st);
+  // counters: words 0-7 the band kernels' queue head and work counters,
+  // 8-10 the exact form's list count, the FP64 band kernel's queue head and
+  // the range words
+  void* cp;
+  if ((rc = ensure(ws, S_COUNTER, 128, &cp, msg))) return rc;
+  unsigned long long* dcount = static_cast<unsigned long long*>(cp);
+  CUDA_TRY(cudaMemsetAsync(dcount, 0, 128, st));
+  unsigned* range = exact ? reinterpret_cast<unsigned*>(dcount + 10) : nullptr;
+  launch_stats(dA, na, m, ultra, sa, st, range);
   launches += 1;
   if (a->has_b) {
     if ((rc = alloc_series(ws, 1, nb, plan.ns_b, &sb, msg))) return rc;
-    launch_stats(dB, nb, m, ultra, sb, st);
+    launch_stats(dB, nb, m, ultra, sb, st, range);
     launches += 1;
   } else {
     sb = sa;
@@ -864,7 +897,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                            int64_t ns_paa, uint64_t* kx, uint64_t* ky) {
       const SeedArgs S{X, Y, paa, ns_paa, kx, ky, excl, m, kl, kSeedFloor, seed_factor(m)};
       const int64_t blocks = std::min<int64_t>((X.ns + 7) / 8, static_cast<int64_t>(ws.sms) * 16);
-      seed_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(S);
+      if (exact)
+        seed_exact_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(S);
+      else
+        seed_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(S);
       ++launches;
     };
     if (plan.self_join) {
@@ -881,14 +917,20 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   // 1NN_INDEX its candidates are verified, for SUM_THRESH the filter
   // threshold is the sum threshold and every cell above it is accumulated).
   // The k-best and matrix-summary types run the FP64 visit kernel.
-  enum { K_FP64, K_MIXED, K_VISIT } kind = visit ? K_VISIT : !mixed ? K_FP64 : K_MIXED;
+  // FP64 1NN joins of some size run the band kernel's exact form.
+  enum { K_FP64, K_MIXED, K_VISIT, K_EXACT } kind =
+      visit ? K_VISIT : mixed ? K_MIXED : exact ? K_EXACT : K_FP64;
+  const bool band = kind == K_MIXED || kind == K_EXACT;  // the FP32 band kernel's geometry
   // (SUM_THRESH keeps the per-cell filter unless asked: its fast path adds
   // the blocks that lie wholly above the threshold, which needs per-cell r)
   const bool coarse = kind == K_MIXED && !is_mat && !is_knn &&
                       (a->filter_mode == 2 ||
                        (a->filter_mode == 0 && is_1nn && m >= kCoarseFilterMinWindow));
+  const bool exact_coarse = kind == K_EXACT && m >= kCoarseFilterMinWindow;
   const void* kfn = kind == K_VISIT ? reinterpret_cast<const void*>(join_visit_kernel)
                   : kind == K_FP64 ? reinterpret_cast<const void*>(join_fp64_kernel)
+                  : exact_coarse ? reinterpret_cast<const void*>(join_exact_1nn_coarse_kernel)
+                  : kind == K_EXACT ? reinterpret_cast<const void*>(join_exact_1nn_kernel)
                   : is_mat ? reinterpret_cast<const void*>(join_mixed_mat_kernel)
                   : is_knn ? reinterpret_cast<const void*>(join_mixed_knn_kernel)
                   : is_1nn ? (coarse ? reinterpret_cast<const void*>(join_mixed_1nn_coarse_kernel)
@@ -897,10 +939,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                                      : reinterpret_cast<const void*>(join_mixed_sum_kernel));
   const int W = kind == K_VISIT ? visit_band_width()
               : kind == K_FP64 ? fp64_band_width() : mixed_1nn_band_width();
-  const int slab = kind == K_MIXED ? mixed_1nn_slab_rows() : fp64_slab_rows();
+  const int slab = band ? mixed_1nn_slab_rows() : fp64_slab_rows();
   const int nthreads = kind == K_VISIT ? visit_threads()
                      : kind == K_FP64 ? fp64_threads() : mixed_1nn_threads();
-  const size_t smem = kind == K_MIXED ? mixed_1nn_smem_bytes() : 0;
+  const size_t smem = band ? mixed_1nn_smem_bytes() : 0;
   if (smem > 0)
     CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
@@ -917,6 +959,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   if (kind == K_MIXED) {
     K = a->anchor_interval > 0 ? a->anchor_interval
                                : (is_1nn ? default_anchor_interval(m) : short_anchor_interval(m));
+  } else if (kind == K_EXACT) {
+    K = default_anchor_interval(m);
   } else {
     K = fp64_segment(m);
   }
@@ -972,7 +1016,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   P.profile_type = is_1nn ? SCAMP_PROFILE_1NN_INDEX : a->profile_type;
   // a join without seeds starts cold: the band kernel refreshes its ring
   // columns' bests every slab (seeded joins start near their final bests)
-  P.refresh_cols = (kind == K_MIXED && ((is_1nn && !seed_a) || knn_mixed)) ? 1 : 0;
+  P.refresh_cols = (band && ((is_1nn && !seed_a) || knn_mixed)) ? 1 : 0;
   P.knn_k = knn_mixed ? static_cast<int>(knn_k) : 0;
   P.threshold = a->distance_threshold;
   P.kl = kl;
@@ -1017,13 +1061,19 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
     if ((rc = ensure(ws, S_PREFIX, prefix.size() * 8, &p, msg))) return rc;
     int64_t* dprefix = static_cast<int64_t*>(p);
     CUDA_TRY(cudaMemcpyAsync(dprefix, prefix.data(), prefix.size() * 8, cudaMemcpyHostToDevice, st));
-    if ((rc = ensure(ws, S_COUNTER, 64, &p, msg))) return rc;
-    CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
     P.band_unit_prefix = dprefix;
-    P.unit_counter = static_cast<unsigned long long*>(p);
-    P.counters = static_cast<unsigned long long*>(p) + 1;
-    P.error_flag = reinterpret_cast<int*>(static_cast<char*>(p) + 48);
-    if (kind == K_MIXED) {
+    P.unit_counter = dcount;
+    P.counters = dcount + 1;
+    P.error_flag = reinterpret_cast<int*>(dcount + 6);
+    if (kind == K_EXACT) {
+      void* q;
+      if ((rc = ensure(ws, S_FP64_LIST, static_cast<size_t>(P.total_units) * 8, &q, msg))) return rc;
+      P.fp64_list = static_cast<int64_t*>(q);
+      P.fp64_count = dcount + 8;
+      P.range = range;
+      P.req_budget = exact_request_budget(K, W);
+    }
+    if (band) {
       // random-walk-like series ask for ~7 (K = 512) to ~18 (K = 1024)
       // 1NN requests per window
       // (k-best lists: a window keeps k candidates open, and cold lists
@@ -1143,6 +1193,22 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
         verify_requests_kernel<<<static_cast<unsigned>(ws.sms * 8), 256, 0, st>>>(P);
         ++launches;
       }
+    } else if (kind == K_EXACT) {
+      if (exact_coarse)
+        join_exact_1nn_coarse_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
+      else
+        join_exact_1nn_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
+      ++launches;
+      if (!nested) {
+        CUDA_TRY(cudaEventRecord(ws.evkv, st));
+        ws.timed_verify = true;
+      }
+      // the units left to FP64 (none in most joins), then the requests
+      JoinParams F = P;
+      F.unit_counter = dcount + 9;
+      join_fp64_kernel<<<static_cast<unsigned>(ws.sms * ws.fp64_occ), fp64_threads(), 0, st>>>(F);
+      verify_exact_kernel<<<static_cast<unsigned>(ws.sms * 8), 256, 0, st>>>(P);
+      launches += 2;
     } else if (kind == K_VISIT) {
       VisitArgs V{};
       V.mode = a->profile_type == SCAMP_PROFILE_APPROX_ALL_NEIGHBORS ? 0 : 1;
@@ -1318,6 +1384,9 @@ int init_workspace(int device, Workspace** out, std::string* msg) {
     CUDA_TRY(cudaEventCreate(&ws.evk0));
     CUDA_TRY(cudaEventCreate(&ws.evk1));
     CUDA_TRY(cudaEventCreate(&ws.evkv));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &ws.fp64_occ, reinterpret_cast<const void*>(join_fp64_kernel), fp64_threads(), 0));
+    ws.fp64_occ = std::max(ws.fp64_occ, 1);
     ws.device = device;
   }
   *out = &ws;
@@ -1991,6 +2060,7 @@ StatsJob batch_stats_job(const BatchArrays& A, int64_t off_n, int64_t off_ns, in
   j.inv32 = A.inv32 + off_ns;
   j.df32 = A.df32 + off_ns;
   j.dg32 = A.dg32 + off_ns;
+  j.range = nullptr;
   return j;
 }
 

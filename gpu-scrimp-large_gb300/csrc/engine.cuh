@@ -75,6 +75,18 @@ __host__ __device__ __forceinline__ int64_t key_to_index(uint64_t key,
   return static_cast<int64_t>(kl.idx_mask - (key & kl.idx_mask));
 }
 
+// Correlation encoded by a profile key, rounded down (a filter threshold may
+// only be lower than the true best).  Integer pipe only.
+__device__ __forceinline__ float key_corr_floor(uint64_t key, const KeyLayout& kl) {
+  const uint64_t q = key >> kl.idx_bits;
+  if (q == 0) return -3.0f;                                 // no match yet
+  const int p = 63 - __clzll(static_cast<long long>(q));    // leading bit
+  const int e = p - kl.frac_bits;                           // (r + 2) in [2^e, 2^(e+1))
+  const uint32_t mant = static_cast<uint32_t>((q << (63 - p)) >> 40) & 0x7FFFFFu;
+  const float v = __uint_as_float((static_cast<uint32_t>(e + 127) << 23) | mant);
+  return v - 2.0f;                                          // exact for v in [1, 4)
+}
+
 // ---------------------------------------------------------------------------
 // Series statistics resident in HBM (one set per input series).
 // ---------------------------------------------------------------------------
@@ -179,7 +191,24 @@ struct JoinParams {
   int64_t rows_per_cell, cols_per_cell;
   uint64_t rpc_magic, cpc_magic;
   int mat_col[kMaxProblems], mat_row[kMaxProblems];
+  // Exact form (FP64 1NN behind the FP32 filter): the range words of the
+  // statistics, the units left to the FP64 band kernel with their count, and
+  // the verification requests a unit may make before it is left to it.  In
+  // the FP64 band kernel a non-null fp64_list makes the units of this list
+  // (two half bands each) its work.
+  const unsigned* range;
+  int64_t* fp64_list;
+  unsigned long long* fp64_count;
+  unsigned req_budget;
 };
+
+// Range within which the exact form's FP32 arithmetic can neither overflow
+// nor lose anything to underflow: |values| <= kExactMaxValue, inverse norms
+// <= kExactMaxInv, their product <= kExactMaxRatio (a cell's FP32 r and its
+// bound then stay finite over any segment).
+constexpr float kExactMaxValue = 1e14f;
+constexpr float kExactMaxInv = 1e15f;
+constexpr float kExactMaxRatio = 1e12f;
 
 // Outputs of the two experimental profile types (join_visit.cu).
 struct VisitArgs {
@@ -242,6 +271,9 @@ struct StatsJob {
   int bshift;
   double *T_clean, *mean, *inv, *df, *dg;
   float *T32, *bhi, *blo, *mu_rel, *inv32, *df32, *dg32;
+  // or null: float bits raised to the largest |T32|, |mu_rel|, |df|, |dg|
+  // and the largest inverse norm of the series (exact form's range check)
+  unsigned* range;
 };
 // Statistics launches: one warp per kStatsChunk windows of a series.
 constexpr int kStatsChunk = 64;
@@ -273,6 +305,10 @@ __global__ void join_mixed_1nn_coarse_kernel(JoinParams P);
 __global__ void join_mixed_sum_coarse_kernel(JoinParams P);
 __global__ void join_mixed_mat_kernel(JoinParams P);  // mixed MATRIX_SUMMARY
 __global__ void join_mixed_knn_kernel(JoinParams P);  // mixed APPROX_ALL_NEIGHBORS
+// FP64 1NN behind the FP32 filter (per-cell and per-step-bound filters)
+__global__ void join_exact_1nn_kernel(JoinParams P);
+__global__ void join_exact_1nn_coarse_kernel(JoinParams P);
+__global__ void verify_exact_kernel(JoinParams P);
 __global__ void verify_requests_kernel(JoinParams P);
 
 // Tensor-core anchors of one problem's chunk of anchor rows (anchor_tc.cu).
@@ -316,10 +352,25 @@ struct SeedArgs {
   float floor;            // pre-pass entries not above it found no partner
   int factor;             // samples per block-averaged sample
 };
+// The partner *j that the pre-pass gives window i of X (false: none).
+__device__ __forceinline__ bool seed_partner(const SeedArgs& S, int64_t i, int64_t* j) {
+  if (i >= S.X.ns) return false;
+  const int64_t ib = i / S.factor;
+  const int64_t ip = ib < S.ns_paa ? ib : S.ns_paa - 1;
+  const uint64_t packed = S.paa[ip];
+  if (!(__uint_as_float(static_cast<uint32_t>(packed)) > S.floor)) return false;  // none found
+  const int64_t p = S.factor * static_cast<int64_t>(packed >> 32) + (i - S.factor * ip);
+  if (p >= S.Y.ns) return false;
+  if (S.excl >= 0 && (p - i < S.excl && i - p < S.excl)) return false;  // trivial match
+  if (isnan(S.X.inv32[i]) || isnan(S.Y.inv32[p])) return false;
+  *j = p;
+  return true;
+}
 __global__ void paa_kernel(const double* __restrict__ T, int64_t n_out, int f,
                            double* __restrict__ out);
 __global__ void fill_floor_kernel(uint64_t* __restrict__ p, int64_t n, float floor);
 __global__ void seed_kernel(SeedArgs S);
+__global__ void seed_exact_kernel(SeedArgs S);  // the seeds' r in FP64
 __global__ void diag_seed_kernel(const Problem* __restrict__ probs,
                                  const int64_t* __restrict__ win_prefix, int nprob, KeyLayout kl);
 

@@ -1,4 +1,6 @@
-// final_eval.cu -- FP64 re-evaluation of every reported 1NN cell.
+// final_eval.cu -- cells evaluated directly in FP64: the re-evaluation of
+// every reported 1NN cell, and the requests and seeds of the double-precision
+// joins that run behind the FP32 filter.
 //
 // Both join forms choose each window's best partner from a recurrence (FP64
 // in the plain form, FP32 behind a filter in the mixed form).  Before the
@@ -71,6 +73,30 @@ __device__ __forceinline__ double corr_group_fp64(const SeriesDev& X, const Seri
     syy += __shfl_xor_sync(0xffffffffu, syy, o);
   }
   return first ? sxy / sqrt(sxx * syy) : 0.0;
+}
+
+// Direct FP64 covariance of window i of X with window j of Y by kLanes lanes,
+// times the two windows' inverse norms; valid in every lane of the group.
+__device__ __forceinline__ double corr_group_norms(const SeriesDev& X, const SeriesDev& Y,
+                                                   int64_t i, int64_t j, int64_t m, int sub) {
+  const double mx = X.mean[i], my = Y.mean[j];
+  const double* __restrict__ tx = X.T + i;
+  const double* __restrict__ ty = Y.T + j;
+  double s0 = 0.0, s1 = 0.0;
+  int64_t t = sub;
+  for (; t + kLanes < m; t += 2 * kLanes) {
+    s0 = fma(tx[t] - mx, ty[t] - my, s0);
+    s1 = fma(tx[t + kLanes] - mx, ty[t + kLanes] - my, s1);
+  }
+  if (t < m) s0 = fma(tx[t] - mx, ty[t] - my, s0);
+  s0 += s1;
+#pragma unroll
+  for (int o = kLanes / 2; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+  return s0 * Y.inv[j] * X.inv[i];
+}
+
+__device__ __forceinline__ uint64_t corr_key(double r, int64_t index, const KeyLayout& kl) {
+  return make_key(q_from_double_bits(__double_as_longlong(r), kl.frac_bits), index, kl);
 }
 
 // The key an input profile entry turns into (profile_to_keys_kernel,
@@ -174,6 +200,58 @@ __global__ void __launch_bounds__(256) knn_final_eval_kernel(EvalSide S, int k, 
         v[p] = x;
       }
       for (int s = 0; s < kc; ++s) list[s] = v[s];
+    }
+  }
+}
+
+// Settles the exact form's requests: every cell that may be its row's or its
+// column's best gets its FP64 r and competes with it.  A request whose upper
+// bound has meanwhile fallen to or below both bests is skipped (decided by
+// the group's first lane: the lanes' loads of a key need not agree).
+__global__ void __launch_bounds__(256) verify_exact_kernel(JoinParams P) {
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (kLanes - 1);
+  const unsigned long long total = P.counters[3];
+  const int64_t n = total < static_cast<unsigned long long>(P.vreq_cap)
+                        ? static_cast<int64_t>(total) : P.vreq_cap;
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  constexpr int kGroups = 32 / kLanes;
+  for (int64_t g0 = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups;
+       g0 < n; g0 += nwarps * kGroups) {
+    const int64_t g = g0 + lane / kLanes;
+    const VerifyReq rq = P.vreq[g < n ? g : g0];
+    const Problem& pr = P.prob[static_cast<int>(rq.i >> 40)];
+    const int64_t i = static_cast<int64_t>(rq.i & ((uint64_t{1} << 40) - 1));
+    const int64_t j = i + rq.d;
+    bool row = g < n && pr.key_row && rq.ub > key_corr_floor(__ldcg(pr.key_row + i), P.kl);
+    bool col = g < n && pr.key_col && rq.ub > key_corr_floor(__ldcg(pr.key_col + j), P.kl);
+    const unsigned open = __ballot_sync(0xffffffffu, sub == 0 && (row || col));
+    if (!open) continue;
+    const bool work = (open >> (lane & ~(kLanes - 1))) & 1u;
+    const double r = corr_group_norms(pr.R, pr.C, i, j, work ? P.m : 0, sub);
+    if (sub == 0 && work && !isnan(r)) {
+      if (row) atomicMax(reinterpret_cast<unsigned long long*>(pr.key_row + i), corr_key(r, j, P.kl));
+      if (col) atomicMax(reinterpret_cast<unsigned long long*>(pr.key_col + j), corr_key(r, i, P.kl));
+    }
+  }
+}
+
+// seed_kernel's seeds with their r in FP64: bests the exact form may rely on.
+__global__ void __launch_bounds__(256) seed_exact_kernel(SeedArgs S) {
+  const int lane = threadIdx.x & 31;
+  const int sub = lane & (kLanes - 1);
+  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  constexpr int kGroups = 32 / kLanes;
+  for (int64_t g0 = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups;
+       g0 < S.X.ns; g0 += nwarps * kGroups) {
+    const int64_t i = g0 + lane / kLanes;
+    int64_t j = 0;
+    const bool work = seed_partner(S, i, &j);
+    const double r = corr_group_norms(S.X, S.Y, work ? i : 0, j, work ? S.m : 0, sub);
+    if (sub == 0 && work && !isnan(r)) {
+      atomicMax(reinterpret_cast<unsigned long long*>(S.key_x + i), corr_key(r, j, S.kl));
+      if (S.key_y)
+        atomicMax(reinterpret_cast<unsigned long long*>(S.key_y + j), corr_key(r, i, S.kl));
     }
   }
 }

@@ -101,19 +101,23 @@ join_fp64_kernel(JoinParams P) {
   const double thr = P.threshold;
   const int64_t ord_thr = ord_double(thr);
   const int64_t K = P.seg_len;
+  // the whole queue, or the half bands of the units the exact form left
+  const bool listed = P.fp64_list != nullptr;
+  const int64_t total_units = listed ? 2 * static_cast<int64_t>(*P.fp64_count) : P.total_units;
 
   for (;;) {
     if (t == 0) sm.unit = static_cast<long long>(atomicAdd(P.unit_counter, 1ull));
     __syncthreads();
     const int64_t u = sm.unit;
     __syncthreads();
-    if (u >= P.total_units) break;
+    if (u >= total_units) break;
 
     int pi;
     int64_t band, ub;
-    decode_unit(P, u, &pi, &band, &ub);
+    decode_unit(P, listed ? P.fp64_list[u >> 1] : u, &pi, &band, &ub);
     const Problem& pr = P.prob[pi];
-    const int64_t D0 = pr.d_lo + band * kBand;
+    const int64_t D0 = pr.d_lo + band * P.band_width + (listed ? (u & 1) * kBand : 0);
+    if (D0 >= pr.d_hi) continue;
     const int64_t rows_b = band_rows(pr.R.ns, pr.C.ns, D0);
     int64_t seg_row[2], seg_len[2];
     seg_row[0] = ub * 2 * K;

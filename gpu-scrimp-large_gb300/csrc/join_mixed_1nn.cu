@@ -1,7 +1,8 @@
 // join_mixed_1nn.cu -- the mixed-precision band kernel: FP32 filter over an
-// FP32 recurrence, exact path for the blocks it flags.  One body, five
-// instantiations: 1NN_INDEX (per-cell and per-step-bound filters),
-// SUM_THRESH, APPROX_ALL_NEIGHBORS (k-best lists) and MATRIX_SUMMARY.
+// FP32 recurrence, exact path for the blocks it flags.  One body:
+// 1NN_INDEX mixed and double (each with a per-cell and a per-step-bound
+// filter), SUM_THRESH, APPROX_ALL_NEIGHBORS (k-best lists) and
+// MATRIX_SUMMARY.
 //
 // Work decomposition as in join_fp64.cu (persistent kernel over a device
 // queue of units = band of kBand diagonals x two row segments of seg_len
@@ -30,6 +31,17 @@
 // cell goes to a request buffer that verify_requests_kernel settles after the
 // join with a direct dot product of the two centred windows.  The k-best
 // form filters at each window's k-th best and inserts into its lists instead.
+//
+// 1NN in double precision (join_exact_1nn_kernel): the same walk, but the
+// FP32 value only rules cells out.  In place of the margin every thread keeps
+// a deterministic bound E on its covariances' error (kStepCov below); a cell
+// whose r + E inv_c inv_r reaches its row's or column's best becomes a
+// request, its lower bound raises the bests, and verify_exact_kernel computes
+// every request that the final bests leave open in FP64.  Nothing FP32 is
+// reported.  The profile is the FP64 kernel's at the FP32 kernel's rate:
+// GB300 issues FP64 at 1/62 of FP32 and both forms cost 4 operations per
+// cell (self-join of 131072 samples, m = 100: 67.5 -> 2.6 ms in the join
+// kernels; 40009 samples with gaps, m = 1024: 39.0 -> 3.4 ms).
 //
 // SUM_THRESH (the reference's sum of every r above the threshold,
 // src/kernels_compute.h:87-113 and 380-392), join_mixed_sum_kernel: every
@@ -90,6 +102,23 @@ constexpr float kStepMarginC = kBoundC * kEps * 2.8284271f * 1.0000153f;
 constexpr float kTrust = 5e-6f;
 constexpr float kNoTarget = 3.0e38f;      // best of a side that is not computed
 
+// The exact form's error bounds (a deterministic bound E on |FP32 covariance
+// - exact covariance| per thread and segment, first order in u = kEps with
+// the factors below covering the higher orders and the bound's own FP32
+// rounding):
+//  - a step of 8 rows: each row rounds twice at no more than the largest
+//    |cov| of the step's start plus the increments so far (16 u max|cov| +
+//    72 u inc), and df, dg are rounded to FP32 (2 u per product, 16 u inc),
+//    inc bounding |df_c dg_r| + |df_r dg_c| over the step's cells;
+//  - an anchor: see anchor_bound().
+// kBoundSlack widens E where it is used (its own sum of up to 2^17 terms
+// rounds by less than 1%); kAbsSlack covers the roundings of r itself and of
+// the comparisons (about 6 u of values within [-3, 1]).
+constexpr float kStepCov = 16.0f * kEps;
+constexpr float kStepInc = 88.0f * kEps;
+constexpr float kBoundSlack = 1.01f;
+constexpr float kAbsSlack = 1.0e-6f;
+
 typedef unsigned long long u64;
 
 __device__ __forceinline__ u64 f2u(float2 v) {
@@ -133,18 +162,6 @@ __device__ __forceinline__ float2 absmax8(const float2 (&c)[8]) {
   return make_float2(fmaxf(x, fabsf(c[7].x)), fmaxf(y, fabsf(c[7].y)));
 }
 
-// Correlation encoded by a profile key, rounded down (a filter threshold may
-// only be lower than the true best).  Integer pipe only.
-__device__ __forceinline__ float key_corr_floor(u64 key, const KeyLayout& kl) {
-  const u64 q = key >> kl.idx_bits;
-  if (q == 0) return -3.0f;                                 // no match yet
-  const int p = 63 - __clzll(static_cast<long long>(q));    // leading bit
-  const int e = p - kl.frac_bits;                           // (r + 2) in [2^e, 2^(e+1))
-  const uint32_t mant = static_cast<uint32_t>((q << (63 - p)) >> 40) & 0x7FFFFFu;
-  const float v = __uint_as_float((static_cast<uint32_t>(e + 127) << 23) | mant);
-  return v - 2.0f;                                          // exact for v in [1, 4)
-}
-
 // A block queued for the exact path: the owner's covariances at the END of
 // the step (the drain rewinds them), the step's drift estimate (largest
 // sum cov^2 over the owner's diagonals plus the increment bound) and the
@@ -183,6 +200,10 @@ struct SlowCtx {
   int64_t rpc, cpc;
   uint64_t rpc_magic, cpc_magic;
   bool mcol, mrow;
+  // exact form: verification requests of the current unit, and whether one
+  // found the buffer full
+  unsigned unit_reqs;
+  unsigned unit_lost;
 };
 
 struct Smem {
@@ -198,7 +219,10 @@ struct Smem {
     struct {
       float2 xr[kAnchorChunk];    // centred row windows of both segments (chunk)
       float2 yc[kYPad];           // column samples (block-relative), padded
-      float2 cb[2][kSpanBlk];     // {bhi, blo} of the blocks of the staged span
+      union {
+        float2 cb[2][kSpanBlk];   // {bhi, blo} of the blocks of the staged span
+        double cbd[2][kSpanBlk];  // exact form: the block offsets in FP64
+      };
     } a;
   } u;
   float2 c_best[kCols];
@@ -235,6 +259,14 @@ __device__ __forceinline__ TableEntry table_entry(float4 f, float2 iv, float2 be
   e.mx = make_float2(fmaxf(0.f, iv.x), fmaxf(0.f, iv.y));
   e.mf = make_float4(fabsf(f.x), fabsf(f.y), fabsf(f.z), fabsf(f.w));
   return e;
+}
+
+// Exact form: dg = (b - mu') + (a - mu) is a rounded sum, off by up to 2^-52
+// of its terms (|dg| + 3 |df| bounds them), which a cancelled |dg| would not
+// show; 2^-20 |df| in its place keeps the step's bound above that.
+__device__ __forceinline__ void floor_dg(TableEntry& e) {
+  e.mf.z = fmaxf(e.mf.z, 9.6e-7f * e.mf.x);
+  e.mf.w = fmaxf(e.mf.w, 9.6e-7f * e.mf.y);
 }
 
 __device__ __forceinline__ void combine(TableEntry& a, const TableEntry& b) {
@@ -593,6 +625,131 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
   return nreq;
 }
 
+// Exact form, one cell per lane that `cand` marks: its FP32 r lies within
+// its error bound mk of a best.  The bests are read again from the profile
+// keys (the staged copies lag behind the other CTAs); a cell that may still
+// win publishes its lower bound r - mk, so the filters rise at once, and
+// asks for its FP64 r.  Called by the whole warp.
+__device__ __forceinline__ void exact_request(Smem& sm, const SlowCtx& cx, bool cand, float rv,
+                                              float mk, int64_t i, int64_t j, int rslot,
+                                              int cslot, int g, int lane, int& nreq) {
+  const Problem& pr = *cx.pr;
+  bool open = false;
+  if (cand) {
+    float fr = kNoTarget, fc = kNoTarget;
+    if (pr.key_row) fr = key_corr_floor(__ldcg(pr.key_row + i), cx.kl);
+    if (pr.key_col) fc = key_corr_floor(__ldcg(pr.key_col + j), cx.kl);
+    open = rv + mk > fr || rv + mk > fc;
+    if (open) {
+      const float lb = rv - mk;
+      const uint64_t q = q_from_float_bits(__float_as_uint(lb), cx.kl.frac_bits);
+      if (lb > -2.f && pr.key_row && lb > fr) {
+        atomicMax(reinterpret_cast<u64*>(pr.key_row + i), make_key(q, j, cx.kl));
+        fr = lb;
+      }
+      if (lb > -2.f && pr.key_col && lb > fc) {
+        atomicMax(reinterpret_cast<u64*>(pr.key_col + j), make_key(q, i, cx.kl));
+        fc = lb;
+      }
+    }
+    // the staged copies only filter: a racing store of a smaller value
+    // costs extra work later, never a wrong result
+    float& rb = g ? sm.r_best[rslot].y : sm.r_best[rslot].x;
+    float& cb = g ? sm.c_best[cslot].y : sm.c_best[cslot].x;
+    if (fr > rb) rb = fr;
+    if (fc > cb) cb = fc;
+  }
+  const unsigned mo = __ballot_sync(0xffffffffu, open);
+  if (!mo) return;
+  const int leader = __ffs(mo) - 1;
+  unsigned long long base = 0;
+  if (lane == leader) {
+    base = atomicAdd(cx.vcount, static_cast<unsigned long long>(__popc(mo)));
+    atomicAdd(&sm.cx.unit_reqs, static_cast<unsigned>(__popc(mo)));
+  }
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (open) {
+    const unsigned long long slot = base + __popc(mo & ((1u << lane) - 1u));
+    ++nreq;
+    if (slot < static_cast<unsigned long long>(cx.vcap)) {
+      VerifyReq rq;
+      rq.i = static_cast<uint64_t>(i) | (static_cast<uint64_t>(cx.prob) << 40);
+      rq.d = static_cast<uint32_t>(j - i);
+      rq.ub = rv + mk;
+      cx.vreq[slot] = rq;
+    } else {
+      sm.cx.unit_lost = 1;  // the FP64 band kernel takes the unit
+    }
+  }
+}
+
+// drain_queue() of the exact form: the same walk (rows last to first, the
+// covariance stepped back over each row), with the deterministic bound.  An
+// item's vw is E at the block's end plus the block's own roundings again,
+// for the steps back.
+__device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane) {
+  __syncwarp();  // the queue was written by other lanes
+  const SlowCtx& cx = sm.cx;
+  const int k = lane & 7;
+  int nreq = 0;
+  for (int p = 0; p < count; p += 4) {
+    const int item = p + (lane >> 3);
+    const bool act = item < count;
+    const SlowItem& it = sm.queue[warp][act ? item : 0];
+    float2 c = it.cov[k];
+    const float2 vw = make_float2(kBoundSlack * it.vw.x, kBoundSlack * it.vw.y);
+    const int s0 = it.s & 255;
+    const int nrows = act ? kRows * ((it.s >> 8) & 255) : 0;
+    const int nrows_w = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(nrows)));
+    const int r0 = s0 * kRows;
+    const int cb0 = 8 * (s0 + it.owner) + k;           // staged column at row 0
+    const int64_t jd = cx.D0 + it.owner * kDiags + k;  // the lane's diagonal
+#pragma unroll 1
+    for (int rw = nrows_w - 1; rw >= 0; --rw) {
+      const bool live = rw < nrows;
+      const int rr = live ? rw : 0;  // rows past the block's end read row 0
+      const int rcs = ringc(cx.ring0, cb0 + rr);
+      const float4 rf = sm.r_fg[r0 + rr];
+      const float4 cf = col_fg(sm, padc(rcs));
+      if (live) {
+        c = fma2(make_float2(-rf.x, -rf.y), make_float2(cf.z, cf.w), c);
+        c = fma2(make_float2(-cf.x, -cf.y), make_float2(rf.z, rf.w), c);
+      }
+      const float2 ivr = sm.r_iv[r0 + rr];
+      const float2 ivc = sm.u.s.c_iv[padc(rcs)];
+      const float2 rv = mul2(mul2(c, ivc), ivr);
+      const float2 mk0 = mul2(mul2(vw, ivc), ivr);
+      const float2 mk = make_float2(mk0.x + kAbsSlack, mk0.y + kAbsSlack);
+      const float2 rb = sm.r_best[r0 + rr];
+      const float2 cbv = sm.c_best[rcs];
+      // (false for NaN: excluded diagonals, windows that cannot match)
+      const bool cx_ = live && rv.x + mk.x > fminf(rb.x, cbv.x);
+      const bool cy_ = live && rv.y + mk.y > fminf(rb.y, cbv.y);
+      if (!__any_sync(0xffffffffu, cx_ || cy_)) continue;
+      const int64_t i0 = cx.rbase[0] + r0 + rr, i1 = cx.rbase[1] + r0 + rr;
+      exact_request(sm, cx, cx_, rv.x, mk.x, i0, i0 + jd, r0 + rr, rcs, 0, lane, nreq);
+      exact_request(sm, cx, cy_, rv.y, mk.y, i1, i1 + jd, r0 + rr, rcs, 1, lane, nreq);
+    }
+  }
+  __syncwarp();
+  return nreq;
+}
+
+// Bound on the error of a thread's FP32 anchors (exact form), per segment,
+// from the squared norms of what it multiplied: x2 of the row window
+// (centred in FP64, rounded once), y2 the sum of T32^2 + d^2 over the column
+// samples y = T32 + d it read (T32 and d rounded once each, so that
+// ||(|T32| + |d| + |y|)|| <= sqrt(8 y2)), and the largest mean difference ek
+// between its windows.  Runs of 32 products, ceil(m / 32) sums of runs and
+// the correction ek * sum x; with ||y|| <= sqrt(8 y2) / 2,
+//   E <= u ||x|| ((35 + m/32) / 2 + 2) sqrt(8 y2) + (38 + m/32) ek sqrt(m))
+// (inputs 1.5 u ||x|| sqrt(8 y2), the rest accumulation).
+__device__ __forceinline__ float anchor_bound(float x2, float y2, float ek, float m) {
+  const float runs = m * (1.f / 32.f);
+  return kBoundSlack * kBoundSlack * kEps * sqrtf(x2) *
+         ((0.5f * (35.f + runs) + 2.f) * sqrtf(8.f * y2) + (38.f + runs) * ek * sqrtf(m));
+}
+
 // SUM_THRESH: the cells of a thread-step that lie within the step's margin
 // m of the threshold (flags fx, fy per segment; rare), walked again by their
 // lane alone from the step's start (rewound from the covariances at its
@@ -759,10 +916,14 @@ __device__ __noinline__ void mat_cells_block(Smem& sm, const float2 (&cov_end)[k
 //          checks every cell with its own r.
 // kMat selects MATRIX_SUMMARY (running grid maxima), kKnn the k-best lists
 // (filters at each window's k-th best); both take the per-cell filter.
-template <bool kSum, bool kCoarse, bool kMat = false, bool kKnn = false>
+// kExact selects the FP64 1NN form: the FP32 arithmetic only rules cells out,
+// by the deterministic bound E (kStepCov ...), and every other cell's r is
+// computed in FP64 (verify_exact_kernel).
+template <bool kSum, bool kCoarse, bool kMat = false, bool kKnn = false, bool kExact = false>
 __device__ __forceinline__ void band_body(const JoinParams& P) {
   static_assert(!(kMat && (kSum || kCoarse)), "the matrix form takes per-cell maxima");
   static_assert(!(kKnn && (kSum || kCoarse || kMat)), "the k-best form is a 1NN variant");
+  static_assert(!(kExact && (kSum || kMat || kKnn)), "the exact form is a 1NN variant");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int t = threadIdx.x;
@@ -795,10 +956,23 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
   }
 
+  // exact form: series out of FP32's safe range leave every unit to the FP64
+  // band kernel
+  bool out_of_range = false;
+  if constexpr (kExact) {
+    const float vmax = __uint_as_float(P.range[0]), imax = __uint_as_float(P.range[1]);
+    out_of_range = !(vmax <= kExactMaxValue && imax <= kExactMaxInv && vmax * imax <= kExactMaxRatio);
+  }
+
   for (;;) {
     if (t == 0) {
       const long long uu = static_cast<long long>(atomicAdd(P.unit_counter, 1ull));
       sm.unit = uu;
+      if constexpr (kExact) {
+        sm.cx.unit_reqs = 0;
+        sm.cx.unit_lost = 0;
+        if (out_of_range && uu < P.total_units) P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = uu;
+      }
       if (uu < P.total_units) {
         int pi;
         int64_t bb, ubb;
@@ -812,6 +986,12 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
     __syncthreads();
     const int64_t u = sm.unit;
     if (u >= P.total_units) break;
+    if constexpr (kExact) {
+      if (out_of_range) {
+        __syncthreads();  // sm.unit is read before the next fetch
+        continue;
+      }
+    }
     const Problem& pr = sm.prob;
     const int64_t K = pr.seg_len;  // per problem: batched joins mix windows
     const int64_t m = pr.m;
@@ -840,6 +1020,10 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
     // row windows and the CTA's column spans are staged in shared memory.
     float2 acc2[kDiags];
     float2 xsum2 = make_float2(0.f, 0.f);
+    // exact form: squared norms of the row window and of the column samples,
+    // and the thread's first window's FP64 mean per segment
+    [[maybe_unused]] float2 x2 = make_float2(0.f, 0.f), y2 = make_float2(0.f, 0.f);
+    [[maybe_unused]] double mu0d[2];
 #pragma unroll
     for (int k = 0; k < kDiags; ++k) acc2[k] = make_float2(0.f, 0.f);
     int64_t jb[2], b0s[2];
@@ -852,6 +1036,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       b0s[g] = jc >> sh;
       mu0[g] = pr.C.mu_rel[jc];   // mu_j0 - boff_c[b0]
       o0[g] = make_float2(pr.C.bhi[b0s[g]], pr.C.blo[b0s[g]]);
+      if constexpr (kExact) mu0d[g] = pr.C.mean[jc];
     }
     const bool live1 = seg_len[1] > 0;
     const int64_t nblk_c = (pr.C.n + (int64_t{1} << sh) - 1) >> sh;
@@ -880,6 +1065,12 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         for (int x = t; x < chunk; x += kThreads) {
           const int64_t p0 = i0 + t0 + x, p1 = i1 + t0 + x;
           float2 v;
+          if constexpr (kExact) {
+            v.x = static_cast<float>(pr.R.T[p0] - pr.R.mean[i0]);
+            v.y = live1 ? static_cast<float>(pr.R.T[p1] - pr.R.mean[i1]) : 0.f;
+            sm.u.a.xr[x] = v;
+            continue;
+          }
           v.x = pr.R.T32[p0] + (block_delta(pr.R, p0 >> sh, bi0) - mr0);
           v.y = live1 ? pr.R.T32[p1] + (block_delta(pr.R, p1 >> sh, bi1) - mr1) : 0.f;
           sm.u.a.xr[x] = v;
@@ -896,7 +1087,8 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
           const int g = t >= kSpanBlk, x = t - g * kSpanBlk;
           const int64_t b = ((g ? cb1 : cb0) >> sh) + x;
           const bool ok = (g == 0 || live1) && b < nblk_c;
-          sm.u.a.cb[g][x] = ok ? make_float2(pr.C.bhi[b], pr.C.blo[b]) : make_float2(0.f, 0.f);
+          if constexpr (kExact) sm.u.a.cbd[g][x] = ok ? pr.C.T[b << sh] : 0.0;
+          else sm.u.a.cb[g][x] = ok ? make_float2(pr.C.bhi[b], pr.C.blo[b]) : make_float2(0.f, 0.f);
         }
         span_b0 = cb0 >> sh;
       }
@@ -920,6 +1112,15 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             // second segment's blocks sit at the same span positions
             cur_b = bf;
             const int x = static_cast<int>(bf - span_b0);
+            if constexpr (kExact) {
+              // in FP64, rounded once
+              dlo.x = (pg < plim0) ? static_cast<float>(sm.u.a.cbd[0][x] - mu0d[0]) : 0.f;
+              dhi.x = (((bf + 1) << sh) < plim0)
+                          ? static_cast<float>(sm.u.a.cbd[0][x + 1] - mu0d[0]) : 0.f;
+              dlo.y = (live1 && pg + K < plim0) ? static_cast<float>(sm.u.a.cbd[1][x] - mu0d[1]) : 0.f;
+              dhi.y = (live1 && ((bf + 1) << sh) + K < plim0)
+                          ? static_cast<float>(sm.u.a.cbd[1][x + 1] - mu0d[1]) : 0.f;
+            } else {
             const float2 l0 = sm.u.a.cb[0][x], h0 = sm.u.a.cb[0][x + 1];
             const float2 l1 = sm.u.a.cb[1][x], h1 = sm.u.a.cb[1][x + 1];
             dlo.x = (pg < plim0) ? ((l0.x - o0[0].x) + (l0.y - o0[0].y)) - mu0[0] : 0.f;
@@ -927,6 +1128,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             dlo.y = (live1 && pg + K < plim0) ? ((l1.x - o0[1].x) + (l1.y - o0[1].y)) - mu0[1] : 0.f;
             dhi.y = (live1 && ((bf + 1) << sh) + K < plim0)
                         ? ((h1.x - o0[1].x) + (h1.y - o0[1].y)) - mu0[1] : 0.f;
+            }
           }
           const int nb = static_cast<int>(((bf + 1) << sh) - pg);  // samples left in block bf
           const int o = pady2(t * kDiags + xg);      // 16-byte aligned slot
@@ -936,6 +1138,20 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             const float4 v = *reinterpret_cast<const float4*>(&sm.u.a.yc[o + q + (q >> 3) * 2]);
             y[q] = make_float2(v.x, v.y);
             y[q + 1] = make_float2(v.z, v.w);
+          }
+          if constexpr (kExact) {
+            // the group's first 8 samples; all 16 in the window's last group
+            const bool last = t0 + xg + 8 >= m;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) y2 = fma2(y[q], y[q], y2);
+            if (last) {
+#pragma unroll
+              for (int q = 8; q < 16; ++q) y2 = fma2(y[q], y[q], y2);
+            }
+            const float2 dm = make_float2(fmaxf(fabsf(dlo.x), fabsf(dhi.x)),
+                                          fmaxf(fabsf(dlo.y), fabsf(dhi.y)));
+            const float cnt = last ? 16.f : 8.f;
+            y2 = fma2(mul2(make_float2(cnt, cnt), dm), dm, y2);
           }
 #pragma unroll
           for (int q = 0; q < 16; ++q) {
@@ -947,6 +1163,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             if (xg + v < c1) {
               const float2 xv = sm.u.a.xr[xg + v];
               xs = make_float2(xs.x + xv.x, xs.y + xv.y);
+              if constexpr (kExact) x2 = fma2(xv, xv, x2);
 #pragma unroll
               for (int k = 0; k < kDiags; ++k) part[k] = fma2(xv, y[v + k], part[k]);
             }
@@ -959,12 +1176,24 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
       __syncthreads();
     }
+    [[maybe_unused]] float2 ekmax = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < kDiags; ++k) {
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
         const int64_t j = jb[g] + k;
         if (tab || j >= pr.C.ns || (g == 1 && !live1)) continue;
+        if constexpr (kExact) {
+          const float e = static_cast<float>(pr.C.mean[j] - mu0d[g]);
+          if (g) {
+            acc2[k].y = fmaf(-e, xsum2.y, acc2[k].y);
+            ekmax.y = fmaxf(ekmax.y, fabsf(e));
+          } else {
+            acc2[k].x = fmaf(-e, xsum2.x, acc2[k].x);
+            ekmax.x = fmaxf(ekmax.x, fabsf(e));
+          }
+          continue;
+        }
         const float ek = (pr.C.mu_rel[j] + block_delta(pr.C, j >> sh, b0s[g])) - mu0[g];
         if (g) acc2[k].y = fmaf(-ek, xsum2.y, acc2[k].y);
         else acc2[k].x = fmaf(-ek, xsum2.x, acc2[k].x);
@@ -982,8 +1211,11 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
     // largest cov^2 among its diagonals (an upper bound of every diagonal's
     // own sum), starting from the anchors' rounding; and the sum of squared
     // increment bounds.
-    float2 Vt;
-    {
+    float2 Vt;  // (the exact form's bound E)
+    if constexpr (kExact) {
+      const float fm = static_cast<float>(m);
+      Vt = make_float2(anchor_bound(x2.x, y2.x, ekmax.x, fm), anchor_bound(x2.y, y2.y, ekmax.y, fm));
+    } else {
       const float2 cm = absmax8(cov);
       Vt = make_float2(pr.anchor_vcoef * cm.x * cm.x, pr.anchor_vcoef * cm.y * cm.y);
     }
@@ -1100,6 +1332,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         }
         sm.c_best[rc] = cbv;
         TableEntry e = table_entry(f, iv, cbv);
+        if constexpr (kExact) floor_dg(e);
         reduce8(e);  // 8 lanes = one aligned ring block
         if ((lane & 7) == 0) {
           const int b = rc >> 3;
@@ -1134,6 +1367,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         sm.r_iv[r] = iv;
         sm.r_best[r] = rbv;
         TableEntry e = table_entry(f, iv, rbv);
+        if constexpr (kExact) floor_dg(e);
         reduce8(e);
         if ((lane & 7) == 0) {
           sm.r_stepmin[r >> 3] = e.mn;
@@ -1171,9 +1405,11 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         const float2 ic0 = sm.c_blkmax_iv[rb], ic1 = sm.c_blkmax_iv[rb + 1];
         const float2 icm = make_float2(fmaxf(ic0.x, ic1.x), fmaxf(ic0.y, ic1.y));
         const float2 irm = sm.r_stepmax_iv[s];
+        [[maybe_unused]] float2 dE = make_float2(0.f, 0.f);  // exact form: the step's share of E
         {
           const float2 cm = absmax8(cov);
-          Vt = fma2(cm, cm, Vt);
+          if constexpr (kExact) dE = mul2(make_float2(kStepCov, kStepCov), cm);
+          else Vt = fma2(cm, cm, Vt);
         }
         {
           // bound of |df_c dg_r| + |df_r dg_c| over the step's cells
@@ -1183,18 +1419,27 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
           const float4 rfm = sm.r_stepmax_fg[s];
           const float2 inc = fma2(make_float2(rfm.x, rfm.y), make_float2(cfm.z, cfm.w),
                                   mul2(make_float2(rfm.z, rfm.w), make_float2(cfm.x, cfm.y)));
-          W = fma2(inc, inc, W);
+          if constexpr (kExact) {
+            dE = fma2(make_float2(kStepInc, kStepInc), inc, dE);
+            Vt = make_float2(Vt.x + dE.x, Vt.y + dE.y);
+          } else {
+            W = fma2(inc, inc, W);
+          }
         }
-        const float vx = Vt.x + W.x, vy = Vt.y + W.y;
+        // (exact form: E with the roundings of the exact path's steps back)
+        const float vx = kExact ? Vt.x + dE.x : Vt.x + W.x;
+        const float vy = kExact ? Vt.y + dE.y : Vt.y + W.y;
         // threshold - margin, the margin as the exact path forms it per cell
         // (C eps sqrt(rows v) inv_c inv_r) but with the block's largest
         // inverse norms, an approximate square root and a 2^-16 allowance
         // for both
-        const float2 mg = mul2(mul2(make_float2(sqrt_approx(vx), sqrt_approx(vy)), icm), irm);
+        const float2 mg = kExact ? mul2(mul2(Vt, icm), irm)
+                                 : mul2(mul2(make_float2(sqrt_approx(vx), sqrt_approx(vy)), icm), irm);
         const float2 tb = sum_mode ? make_float2(thr, thr)
                                    : make_float2(fminf(bm.x, rsm.x), fminf(bm.y, rsm.y));
-        const float2 tt = fma2(make_float2(-kStepMarginC, -kStepMarginC), mg, tb);
-        const float tx = tt.x, ty = tt.y;
+        constexpr float kMg = kExact ? kBoundSlack : kStepMarginC;
+        const float2 tt = fma2(make_float2(-kMg, -kMg), mg, tb);
+        const float tx = kExact ? tt.x - kAbsSlack : tt.x, ty = kExact ? tt.y - kAbsSlack : tt.y;
 
         // fast path: recurrence + block maximum
         float bx = -3.f, by = -3.f;
@@ -1471,7 +1716,13 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             n_slow += trig ? 1u : 0u;
           }
         }
-        vlast = make_float2(vx, vy);
+        if constexpr (kExact) {
+          // the bound of a block that starts in the pair's first step: E at
+          // its end plus both steps' roundings for the steps back
+          vlast = P == 0 ? dE : make_float2(vx + vlast.x, vy + vlast.y);
+        } else {
+          vlast = make_float2(vx, vy);
+        }
       };
 #pragma unroll 1
       for (int s = 0; s < kSteps; s += 2) {
@@ -1492,7 +1743,8 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         const unsigned pmask = __ballot_sync(0xffffffffu, pend >= 0);
         if (pmask || qn >= kQueue / 2 || (qn && s + 2 == kSteps)) {
           if (qn) {
-            n_verify += drain_queue<!kCoarse>(sm, warp, qn, lane);
+            n_verify += kExact ? drain_exact(sm, warp, qn, lane)
+                               : drain_queue<!kCoarse>(sm, warp, qn, lane);
             qn = 0;
           }
           const int np = __popc(pmask);
@@ -1507,13 +1759,26 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
               it.owner = t;
             }
             const int take = (np - done) < kQueue ? (np - done) : kQueue;
-            n_verify += drain_queue<!kCoarse>(sm, warp, take, lane);
+            n_verify += kExact ? drain_exact(sm, warp, take, lane)
+                               : drain_queue<!kCoarse>(sm, warp, take, lane);
           }
           pend = -1;
         }
       }
       n_steps += kSteps;
       __syncthreads();
+      if constexpr (kExact) {
+        // A unit whose cells its FP32 values cannot rule out (error bounds
+        // above the spread of the correlations: near-flat windows beside
+        // large steps, exact repeats everywhere) is left to the FP64 band
+        // kernel; what it published stands.
+        const bool leave = sm.cx.unit_reqs > P.req_budget || sm.cx.unit_lost;
+        __syncthreads();
+        if (leave) {
+          if (t == 0) P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = u;
+          break;
+        }
+      }
       if (sum_mode && pr.sum_row) {
         // the slab's row sums (thread t: row t; it restages row t next)
         const float2 v = sm.r_best[t];
@@ -1588,6 +1853,14 @@ __global__ void __launch_bounds__(kThreads, 4) join_mixed_1nn_coarse_kernel(Join
 
 __global__ void __launch_bounds__(kThreads, 4) join_mixed_sum_coarse_kernel(JoinParams P) {
   band_body<true, true>(P);
+}
+
+__global__ void __launch_bounds__(kThreads, 4) join_exact_1nn_kernel(JoinParams P) {
+  band_body<false, false, false, false, true>(P);
+}
+
+__global__ void __launch_bounds__(kThreads, 4) join_exact_1nn_coarse_kernel(JoinParams P) {
+  band_body<false, true, false, false, true>(P);
 }
 
 // Settles the verification requests of the band kernels, one warp per
@@ -1699,15 +1972,9 @@ __global__ void __launch_bounds__(256) seed_kernel(SeedArgs S) {
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
   for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
        i < S.X.ns; i += nwarps) {
-    const int64_t ib = i / S.factor;
-    const int64_t ip = ib < S.ns_paa ? ib : S.ns_paa - 1;
-    const uint64_t packed = S.paa[ip];
-    if (!(__uint_as_float(static_cast<uint32_t>(packed)) > S.floor)) continue;  // no partner found
-    const int64_t j = S.factor * static_cast<int64_t>(packed >> 32) + (i - S.factor * ip);
-    if (j >= S.Y.ns) continue;
-    if (S.excl >= 0 && (j - i < S.excl && i - j < S.excl)) continue;  // trivial match
+    int64_t j;
+    if (!seed_partner(S, i, &j)) continue;
     const float ivx = S.X.inv32[i], ivy = S.Y.inv32[j];
-    if (isnan(ivx) || isnan(ivy)) continue;
     const float cv = verify_cov_warp(S.X, S.Y, i, j, S.m, lane);
     if (lane == 0) {
       const uint64_t q = q_from_float_bits(__float_as_uint((cv * ivy) * ivx), S.kl.frac_bits);

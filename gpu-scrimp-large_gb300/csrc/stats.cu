@@ -51,8 +51,9 @@ __device__ __forceinline__ void add2(double& s, double& c, double s2, double c2)
 struct StatsOut {
   double *mean, *inv, *df, *dg;
   float *mu_rel, *inv32, *df32, *dg32;
+  float vmax, imax;  // the lane's largest |value| and inverse norm
 };
-__device__ __forceinline__ void write_window(const StatsOut& o, int64_t w, double x_out, double x_in,
+__device__ __forceinline__ void write_window(StatsOut& o, int64_t w, double x_out, double x_in,
                                              bool has_next, double mu, double mu_lo, double mu_next,
                                              double mu_next_lo, double ssd, bool nan_window,
                                              double block_off) {
@@ -62,14 +63,18 @@ __device__ __forceinline__ void write_window(const StatsOut& o, int64_t w, doubl
     f = (x_in - x_out) / 2.0;
     g = ((x_in - mu_next) - mu_next_lo) + ((x_out - mu) - mu_lo);
   }
+  const float mr = static_cast<float>((mu - block_off) + mu_lo);
+  const float iv32 = static_cast<float>(iv), f32 = static_cast<float>(f), g32 = static_cast<float>(g);
   o.mean[w] = mu;
-  o.mu_rel[w] = static_cast<float>((mu - block_off) + mu_lo);
+  o.mu_rel[w] = mr;
   o.inv[w] = iv;
   o.df[w] = f;
   o.dg[w] = g;
-  o.inv32[w] = static_cast<float>(iv);
-  o.df32[w] = static_cast<float>(f);
-  o.dg32[w] = static_cast<float>(g);
+  o.inv32[w] = iv32;
+  o.df32[w] = f32;
+  o.dg32[w] = g32;
+  o.vmax = fmaxf(fmaxf(o.vmax, fabsf(mr)), fmaxf(fabsf(f32), fabsf(g32)));
+  o.imax = fmaxf(o.imax, iv32);  // NaN (no match possible) does not count
 }
 
 // Statistics of windows [chunk * kStatsChunk, (chunk + 1) * kStatsChunk) of
@@ -90,7 +95,7 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
                                            int64_t n, int64_t m, int ultra, int bshift,
                                            double* __restrict__ T_clean, float* __restrict__ T32,
                                            float* __restrict__ bhi, float* __restrict__ blo,
-                                           const StatsOut& o) {
+                                           StatsOut& o) {
   constexpr unsigned kAll = 0xffffffffu;
   const int64_t ns = n - m + 1;
   const int64_t w0 = chunk * kStatsChunk;
@@ -107,7 +112,9 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
       T_clean[t] = c;
       const int64_t b = t >> bshift;
       const double off = block_off(b);
-      T32[t] = static_cast<float>(c - off);
+      const float rel = static_cast<float>(c - off);
+      T32[t] = rel;
+      o.vmax = fmaxf(o.vmax, fabsf(rel));
       if ((b << bshift) == t) {
         const float hi = static_cast<float>(off);
         bhi[b] = hi;
@@ -262,9 +269,18 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
 
 __global__ void __launch_bounds__(kStatsThreads) stats_kernel(StatsJob j, int ultra) {
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * kStatsThreads + threadIdx.x) >> 5;
-  const StatsOut o{j.mean, j.inv, j.df, j.dg, j.mu_rel, j.inv32, j.df32, j.dg32};
+  StatsOut o{j.mean, j.inv, j.df, j.dg, j.mu_rel, j.inv32, j.df32, j.dg32, 0.f, 0.f};
   stats_body(warp, threadIdx.x & 31, j.T_raw, j.n, j.m, ultra, j.bshift, j.T_clean, j.T32, j.bhi,
              j.blo, o);
+  if (j.range) {
+    // non-negative floats order as their bits (an infinity counts as such)
+    const unsigned v = __reduce_max_sync(0xffffffffu, __float_as_uint(o.vmax));
+    const unsigned i = __reduce_max_sync(0xffffffffu, __float_as_uint(o.imax));
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(j.range, v);
+      atomicMax(j.range + 1, i);
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kStatsThreads)
@@ -278,7 +294,7 @@ stats_batch_kernel(const StatsJob* __restrict__ jobs, const int64_t* __restrict_
   }
   const StatsJob& j = jobs[lo];
   const int64_t warp = ((b - block_prefix[lo]) * kStatsThreads + threadIdx.x) >> 5;
-  const StatsOut o{j.mean, j.inv, j.df, j.dg, j.mu_rel, j.inv32, j.df32, j.dg32};
+  StatsOut o{j.mean, j.inv, j.df, j.dg, j.mu_rel, j.inv32, j.df32, j.dg32, 0.f, 0.f};
   stats_body(warp, threadIdx.x & 31, j.T_raw, j.n, j.m, 0, j.bshift, j.T_clean, j.T32, j.bhi, j.blo,
              o);
 }
