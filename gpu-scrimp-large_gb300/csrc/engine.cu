@@ -125,14 +125,25 @@ int64_t cold_anchor_interval(int64_t m) {
   return std::min<int64_t>(std::max<int64_t>(4096, 2 * m), std::max<int64_t>(1024, 8 * m));
 }
 
-// The exact form serves FP64 1NN joins of at least this many cells: smaller
-// ones spend their time raising bests from nothing, every step flagged
-// (whole join, FP64 band kernel against exact form: 6001 samples, m = 33,
-// 0.33 / 0.68 ms; 15000 samples, m = 64, 1.64 / 0.73 ms).
-constexpr uint64_t kExactMinCells = uint64_t{1} << 25;
+// The exact form serves FP64 1NN joins of at least this many cells: below,
+// its launches and the latency of its units cost more than the FP64 kernel
+// (device time, exact / FP64: 4000 samples 0.21-0.32 / 0.25-0.31 ms, 6000
+// 0.21-0.33 / 0.31-0.43, 12000 0.22-0.32 / 0.89-1.45; m = 32 and 100).
+constexpr uint64_t kExactMinCells = 12000000;
 // Its longest window: the FP32 bounds are first order in m 2^-24, and the
 // rounding of their own sums is covered up to here.
 constexpr int64_t kExactMaxWindow = 65536;
+
+// Segment length of an exact join that is too small for its anchor interval:
+// units for v waves of resident CTAs.  A unit costs m FMAs per diagonal for
+// its anchors and about 3 per cell, and the last wave is half empty, so the
+// time goes as (v + 1/2) (m + 3 K_1 / v), K_1 the rows of one wave's units:
+// least at v = sqrt(3 K_1 / 2 m).
+int64_t exact_segment(double cells, int64_t resident, int W, int slab, int64_t m) {
+  const double k1 = cells / (2.0 * W * static_cast<double>(resident));
+  const double v = std::min(8.0, std::max(3.0, std::sqrt(1.5 * k1 / static_cast<double>(m))));
+  return (static_cast<int64_t>(k1 / v) / slab + 1) * slab;
+}
 
 // Verification requests a unit of the exact form may make before the FP64
 // band kernel takes it: one for every fourth cell.  A request costs the FP64
@@ -484,6 +495,21 @@ void launch_stats(const double* raw, int64_t n, int64_t m, bool ultra, const Ser
   stats_kernel<<<static_cast<unsigned>(stats_blocks(n - m + 1)), kStatsThreads, 0, st>>>(j, ultra ? 1 : 0);
 }
 
+// The bounds pass over the units of P (its own queue head).
+int launch_bounds(const JoinParams& P, bool exact, int64_t grid, size_t smem, cudaStream_t st,
+                  std::string* msg) {
+  const void* fn = exact ? reinterpret_cast<const void*>(bound_exact_1nn_kernel)
+                         : reinterpret_cast<const void*>(bound_mixed_1nn_kernel);
+  CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(smem)));
+  if (exact)
+    bound_exact_1nn_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
+  else
+    bound_mixed_1nn_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
+  CUDA_TRY(cudaGetLastError());
+  return SCAMP_OK;
+}
+
 // One problem's chunk of tensor-core anchors: anchor rows s0 .. s0 + nrows
 // - 1 of the row series against every diagonal of the problem, into `table`
 // (nrows x wp_pad floats, the layout of anchor_tc.cu).
@@ -770,7 +796,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   NvtxRange nvtx_join(nested ? "seeding pre-pass join" : "join");
   uint64_t *seed_a = nullptr, *seed_b = nullptr;
   int64_t seed_ns_a = 0, seed_ns_b = 0;
-  if (!nested && (mixed || exact) && is_1nn && seedable(a, plan)) {
+  if (!nested && mixed && is_1nn && seedable(a, plan)) {
     if ((rc = seed_prepass(ws, a, plan, dA, dB, st, &seed_a, &seed_b, &seed_ns_a, &seed_ns_b,
                            &launches, msg)))
       return rc;
@@ -782,8 +808,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   sa.bshift = sb.bshift = block_shift(m);
   if ((rc = alloc_series(ws, 0, na, plan.ns_a, &sa, msg))) return rc;
   // counters: words 0-7 the band kernels' queue head and work counters,
-  // 8-10 the exact form's list count, the FP64 band kernel's queue head and
-  // the range words
+  // 8-11 the exact form's list count, the FP64 band kernel's queue head, the
+  // range words and the bounds pass's queue head
   void* cp;
   if ((rc = ensure(ws, S_COUNTER, 128, &cp, msg))) return rc;
   unsigned long long* dcount = static_cast<unsigned long long*>(cp);
@@ -897,10 +923,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                            int64_t ns_paa, uint64_t* kx, uint64_t* ky) {
       const SeedArgs S{X, Y, paa, ns_paa, kx, ky, excl, m, kl, kSeedFloor, seed_factor(m)};
       const int64_t blocks = std::min<int64_t>((X.ns + 7) / 8, static_cast<int64_t>(ws.sms) * 16);
-      if (exact)
-        seed_exact_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(S);
-      else
-        seed_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(S);
+      seed_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(S);
       ++launches;
     };
     if (plan.self_join) {
@@ -926,10 +949,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   const bool coarse = kind == K_MIXED && !is_mat && !is_knn &&
                       (a->filter_mode == 2 ||
                        (a->filter_mode == 0 && is_1nn && m >= kCoarseFilterMinWindow));
-  const bool exact_coarse = kind == K_EXACT && m >= kCoarseFilterMinWindow;
   const void* kfn = kind == K_VISIT ? reinterpret_cast<const void*>(join_visit_kernel)
                   : kind == K_FP64 ? reinterpret_cast<const void*>(join_fp64_kernel)
-                  : exact_coarse ? reinterpret_cast<const void*>(join_exact_1nn_coarse_kernel)
                   : kind == K_EXACT ? reinterpret_cast<const void*>(join_exact_1nn_kernel)
                   : is_mat ? reinterpret_cast<const void*>(join_mixed_mat_kernel)
                   : is_knn ? reinterpret_cast<const void*>(join_mixed_knn_kernel)
@@ -964,7 +985,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   } else {
     K = fp64_segment(m);
   }
-  K = std::min(K, std::max<int64_t>(k_lb, slab));
+  if (kind == K_EXACT)
+    K = std::min(K, exact_segment(cells_d, resident, W, slab, m));
+  else
+    K = std::min(K, std::max<int64_t>(k_lb, slab));
   K = std::max<int64_t>(slab, (K / slab) * slab);
   {
     // The mixed 1NN kernel pairs the two segments of a unit; their column
@@ -1094,6 +1118,13 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       CUDA_TRY(cudaEventRecord(ws.evk0, st));
       ws.timed_kernel = true;
     }
+    // ---- bounds pass: joins without seeds start from lower bounds ----
+    if ((kind == K_EXACT || (kind == K_MIXED && is_1nn)) && !seed_a && !use_tc) {
+      JoinParams B = P;
+      B.unit_counter = dcount + 11;
+      if ((rc = launch_bounds(B, exact, grid, smem, st, msg))) return rc;
+      ++launches;
+    }
     auto launch_band = [&](const JoinParams& Q, int64_t g) {
       if (is_mat)
         join_mixed_mat_kernel<<<static_cast<unsigned>(g), nthreads, smem, st>>>(Q);
@@ -1194,10 +1225,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
         ++launches;
       }
     } else if (kind == K_EXACT) {
-      if (exact_coarse)
-        join_exact_1nn_coarse_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
-      else
-        join_exact_1nn_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
+      join_exact_1nn_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
       ++launches;
       if (!nested) {
         CUDA_TRY(cudaEventRecord(ws.evkv, st));

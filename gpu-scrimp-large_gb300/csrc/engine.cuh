@@ -305,10 +305,11 @@ __global__ void join_mixed_1nn_coarse_kernel(JoinParams P);
 __global__ void join_mixed_sum_coarse_kernel(JoinParams P);
 __global__ void join_mixed_mat_kernel(JoinParams P);  // mixed MATRIX_SUMMARY
 __global__ void join_mixed_knn_kernel(JoinParams P);  // mixed APPROX_ALL_NEIGHBORS
-// FP64 1NN behind the FP32 filter (per-cell and per-step-bound filters)
-__global__ void join_exact_1nn_kernel(JoinParams P);
-__global__ void join_exact_1nn_coarse_kernel(JoinParams P);
+__global__ void join_exact_1nn_kernel(JoinParams P);  // FP64 1NN behind the FP32 filter
 __global__ void verify_exact_kernel(JoinParams P);
+// Lower bounds of every window's best before the join itself (FP64 / mixed)
+__global__ void bound_exact_1nn_kernel(JoinParams P);
+__global__ void bound_mixed_1nn_kernel(JoinParams P);
 __global__ void verify_requests_kernel(JoinParams P);
 
 // Tensor-core anchors of one problem's chunk of anchor rows (anchor_tc.cu).
@@ -352,25 +353,10 @@ struct SeedArgs {
   float floor;            // pre-pass entries not above it found no partner
   int factor;             // samples per block-averaged sample
 };
-// The partner *j that the pre-pass gives window i of X (false: none).
-__device__ __forceinline__ bool seed_partner(const SeedArgs& S, int64_t i, int64_t* j) {
-  if (i >= S.X.ns) return false;
-  const int64_t ib = i / S.factor;
-  const int64_t ip = ib < S.ns_paa ? ib : S.ns_paa - 1;
-  const uint64_t packed = S.paa[ip];
-  if (!(__uint_as_float(static_cast<uint32_t>(packed)) > S.floor)) return false;  // none found
-  const int64_t p = S.factor * static_cast<int64_t>(packed >> 32) + (i - S.factor * ip);
-  if (p >= S.Y.ns) return false;
-  if (S.excl >= 0 && (p - i < S.excl && i - p < S.excl)) return false;  // trivial match
-  if (isnan(S.X.inv32[i]) || isnan(S.Y.inv32[p])) return false;
-  *j = p;
-  return true;
-}
 __global__ void paa_kernel(const double* __restrict__ T, int64_t n_out, int f,
                            double* __restrict__ out);
 __global__ void fill_floor_kernel(uint64_t* __restrict__ p, int64_t n, float floor);
 __global__ void seed_kernel(SeedArgs S);
-__global__ void seed_exact_kernel(SeedArgs S);  // the seeds' r in FP64
 __global__ void diag_seed_kernel(const Problem* __restrict__ probs,
                                  const int64_t* __restrict__ win_prefix, int nprob, KeyLayout kl);
 

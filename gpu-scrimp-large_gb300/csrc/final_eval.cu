@@ -1,6 +1,6 @@
 // final_eval.cu -- cells evaluated directly in FP64: the re-evaluation of
-// every reported 1NN cell, and the requests and seeds of the double-precision
-// joins that run behind the FP32 filter.
+// every reported 1NN cell, and the requests of the double-precision joins that
+// run behind the FP32 filter.
 //
 // Both join forms choose each window's best partner from a recurrence (FP64
 // in the plain form, FP32 behind a filter in the mixed form).  Before the
@@ -232,26 +232,6 @@ __global__ void __launch_bounds__(256) verify_exact_kernel(JoinParams P) {
     if (sub == 0 && work && !isnan(r)) {
       if (row) atomicMax(reinterpret_cast<unsigned long long*>(pr.key_row + i), corr_key(r, j, P.kl));
       if (col) atomicMax(reinterpret_cast<unsigned long long*>(pr.key_col + j), corr_key(r, i, P.kl));
-    }
-  }
-}
-
-// seed_kernel's seeds with their r in FP64: bests the exact form may rely on.
-__global__ void __launch_bounds__(256) seed_exact_kernel(SeedArgs S) {
-  const int lane = threadIdx.x & 31;
-  const int sub = lane & (kLanes - 1);
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  constexpr int kGroups = 32 / kLanes;
-  for (int64_t g0 = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups;
-       g0 < S.X.ns; g0 += nwarps * kGroups) {
-    const int64_t i = g0 + lane / kLanes;
-    int64_t j = 0;
-    const bool work = seed_partner(S, i, &j);
-    const double r = corr_group_norms(S.X, S.Y, work ? i : 0, j, work ? S.m : 0, sub);
-    if (sub == 0 && work && !isnan(r)) {
-      atomicMax(reinterpret_cast<unsigned long long*>(S.key_x + i), corr_key(r, j, S.kl));
-      if (S.key_y)
-        atomicMax(reinterpret_cast<unsigned long long*>(S.key_y + j), corr_key(r, i, S.kl));
     }
   }
 }
