@@ -125,35 +125,34 @@ int64_t cold_anchor_interval(int64_t m) {
   return std::min<int64_t>(std::max<int64_t>(4096, 2 * m), std::max<int64_t>(1024, 8 * m));
 }
 
-// The exact form serves FP64 1NN joins of at least this many cells: below,
-// its launches and the latency of its units cost more than the FP64 kernel
-// (device time, exact / FP64: 4000 samples 0.21-0.32 / 0.25-0.31 ms, 6000
-// 0.21-0.33 / 0.31-0.43, 12000 0.22-0.32 / 0.89-1.45; m = 32 and 100).
-constexpr uint64_t kExactMinCells = 12000000;
-// Its longest window: the FP32 bounds are first order in m 2^-24, and the
-// rounding of their own sums is covered up to here.
+// Longest window of the exact form (which serves FP64 1NN joins of every
+// size: device time of whole joins, FP64 band kernel / exact form, 500
+// samples m = 32 0.24 / 0.17 ms, 4000 m = 100 0.32 / 0.18): its FP32 bounds are
+// first order in m 2^-24, and the rounding of their own sums is covered up to
+// here.
 constexpr int64_t kExactMaxWindow = 65536;
 
 // Segment length of an exact join that is too small for its anchor interval:
 // units for v waves of resident CTAs.  A unit costs m FMAs per diagonal for
 // its anchors and about 3 per cell, and the last wave is half empty, so the
 // time goes as (v + 1/2) (m + 3 K_1 / v), K_1 the rows of one wave's units:
-// least at v = sqrt(3 K_1 / 2 m).
+// least at v = sqrt(3 K_1 / 2 m).  Whole slabs, or a fraction of one where
+// the join has fewer units than resident CTAs.
 int64_t exact_segment(double cells, int64_t resident, int W, int slab, int64_t m) {
   const double k1 = cells / (2.0 * W * static_cast<double>(resident));
+  if (k1 < slab) return (static_cast<int64_t>(k1) / 32 + 1) * 32;
   const double v = std::min(8.0, std::max(3.0, std::sqrt(1.5 * k1 / static_cast<double>(m))));
   return (static_cast<int64_t>(k1 / v) / slab + 1) * slab;
 }
 
 // Verification requests a unit of the exact form may make before the FP64
-// band kernel takes it: one for every fourth cell.  A request costs the FP64
-// pipe 3 m operations against 4 for a cell of the FP64 kernel, but most are
-// ruled out by the final bests before that: joins that start cold make up to
-// a hundred per window (30000 samples, m = 1024: 3.2 ms with this budget,
-// 7.4 ms with one request per 12 cells).
-unsigned exact_request_budget(int64_t K, int W) {
-  return static_cast<unsigned>(2 * K * W / 4);
-}
+// band kernel takes it, per cell of the unit.  Near-ties may ask for many
+// (most are ruled out by the final bests before FP64 computes them: 30000
+// samples, m = 1024, 3.2 ms with one request per four cells, 7.4 ms with
+// one per 12).  Requests of wide bounds come by the million where a spike or
+// a flat stretch leaves FP32 nothing, so a few say that the unit is lost.
+constexpr int64_t kReqPerCells = 4;
+constexpr int64_t kWidePerCells = 1024;
 
 // Rows between seeds of the FP64 form.  The FP64 recurrence drifts by
 // ~2^-53 per row, so seeds only bound the work lost to them: 32 m rows keep
@@ -790,7 +789,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   // FP64 1NN joins on the mixed band kernel: cells that deterministic bounds
   // cannot rule out get their FP64 r, so the profile is the FP64 one
   const bool exact = is_1nn && a->precision_type == SCAMP_PRECISION_DOUBLE && !nested &&
-                     plan.cells >= kExactMinCells && m <= kExactMaxWindow;
+                     m <= kExactMaxWindow;
 
   // ---- seeds: block-averaged pre-pass (mixed 1NN joins that pay for it) ----
   NvtxRange nvtx_join(nested ? "seeding pre-pass join" : "join");
@@ -985,11 +984,12 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   } else {
     K = fp64_segment(m);
   }
-  if (kind == K_EXACT)
+  if (kind == K_EXACT) {
     K = std::min(K, exact_segment(cells_d, resident, W, slab, m));
-  else
+  } else {
     K = std::min(K, std::max<int64_t>(k_lb, slab));
-  K = std::max<int64_t>(slab, (K / slab) * slab);
+    K = std::max<int64_t>(slab, (K / slab) * slab);
+  }
   {
     // The mixed 1NN kernel pairs the two segments of a unit; their column
     // spans must be a whole number of FP32-copy blocks apart.
@@ -1095,7 +1095,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       P.fp64_list = static_cast<int64_t*>(q);
       P.fp64_count = dcount + 8;
       P.range = range;
-      P.req_budget = exact_request_budget(K, W);
+      P.req_budget = static_cast<unsigned>(2 * K * W / kReqPerCells);
+      P.wide_budget = static_cast<unsigned>(2 * K * W / kWidePerCells);
     }
     if (band) {
       // random-walk-like series ask for ~7 (K = 512) to ~18 (K = 1024)

@@ -199,7 +199,7 @@ struct JoinParams {
   const unsigned* range;
   int64_t* fp64_list;
   unsigned long long* fp64_count;
-  unsigned req_budget;
+  unsigned req_budget, wide_budget;  // all of them, those of wide bounds
 };
 
 // Range within which the exact form's FP32 arithmetic can neither overflow

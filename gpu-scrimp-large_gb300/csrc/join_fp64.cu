@@ -101,9 +101,22 @@ join_fp64_kernel(JoinParams P) {
   const double thr = P.threshold;
   const int64_t ord_thr = ord_double(thr);
   const int64_t K = P.seg_len;
-  // the whole queue, or the half bands of the units the exact form left
+  // The whole queue, or the units the exact form left: each in half bands
+  // (its bands are twice as wide), and where they are too few for the
+  // resident CTAs also in pieces of its rows (a CTA alone on an SM runs at a
+  // quarter of the SM's FP64 rate: a handful of units of 1024 rows took 4.3
+  // ms), each of at least 128 rows and m, which bounds the work of its seeds.
   const bool listed = P.fp64_list != nullptr;
-  const int64_t total_units = listed ? 2 * static_cast<int64_t>(*P.fp64_count) : P.total_units;
+  int64_t pieces = 1, piece_len = K, total_units = P.total_units;
+  if (listed) {
+    const int64_t left = static_cast<int64_t>(*P.fp64_count);
+    const int64_t least = P.m > 128 ? P.m : 128;
+    if (left > 0) pieces = gridDim.x / (2 * left);
+    if (pieces > K / least) pieces = K / least;
+    if (pieces < 1) pieces = 1;
+    piece_len = ((K + pieces - 1) / pieces + kSlab - 1) / kSlab * kSlab;
+    total_units = 2 * left * pieces;
+  }
 
   for (;;) {
     if (t == 0) sm.unit = static_cast<long long>(atomicAdd(P.unit_counter, 1ull));
@@ -114,17 +127,19 @@ join_fp64_kernel(JoinParams P) {
 
     int pi;
     int64_t band, ub;
-    decode_unit(P, listed ? P.fp64_list[u >> 1] : u, &pi, &band, &ub);
+    const int64_t half = u / pieces, row_off = (u - half * pieces) * piece_len;
+    decode_unit(P, listed ? P.fp64_list[half >> 1] : u, &pi, &band, &ub);
     const Problem& pr = P.prob[pi];
-    const int64_t D0 = pr.d_lo + band * P.band_width + (listed ? (u & 1) * kBand : 0);
+    const int64_t D0 = pr.d_lo + band * P.band_width + (listed ? (half & 1) * kBand : 0);
     if (D0 >= pr.d_hi) continue;
     const int64_t rows_b = band_rows(pr.R.ns, pr.C.ns, D0);
     int64_t seg_row[2], seg_len[2];
-    seg_row[0] = ub * 2 * K;
+    seg_row[0] = ub * 2 * K + row_off;
     seg_row[1] = seg_row[0] + K;
+    const int64_t most = K - row_off < piece_len ? K - row_off : piece_len;
     for (int g = 0; g < 2; ++g) {
       int64_t l = rows_b - seg_row[g];
-      seg_len[g] = l < 0 ? 0 : (l > K ? K : l);
+      seg_len[g] = l < 0 ? 0 : (l > most ? most : l);
     }
     const int64_t d_my = D0 + t * kDiags;
 

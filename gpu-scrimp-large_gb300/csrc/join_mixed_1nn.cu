@@ -101,6 +101,7 @@ constexpr int kYPad = (kYSpan / 8) * 10;              // padded: 10 pairs per 8
 // blocks hold >= 32 samples: the span plus the block after its end
 constexpr int kSpanBlk = kYSpan / 32 + 3;
 constexpr int kQueue = 16;                // queued blocks per warp
+constexpr int kReqChunk = 64;             // request slots a warp takes at a time (exact form)
 constexpr float kEps = 5.9604645e-8f;     // 2^-24
 constexpr float kBoundC = 4.0f;
 // kBoundC * kEps * sqrt(kRows), widened by 2^-16 (see the step's threshold)
@@ -129,6 +130,9 @@ constexpr float kStepCov = 16.0f * kEps;
 constexpr float kStepInc = 88.0f * kEps;
 constexpr float kBoundSlack = 1.01f;
 constexpr float kAbsSlack = 1.0e-6f;
+// A request whose bound is wider says that FP32 carries nothing there (a
+// large step has passed through the windows); JoinParams::wide_budget.
+constexpr float kWideBound = 1.0f / 8.0f;
 // Mixed form: how far below the FP32 values its bounds pass stays.  Wider
 // than any error of a trusted value, so that a cell near a window's best is
 // still settled by the join itself, as in a join that starts from nothing.
@@ -215,10 +219,12 @@ struct SlowCtx {
   int64_t rpc, cpc;
   uint64_t rpc_magic, cpc_magic;
   bool mcol, mrow;
-  // exact form: verification requests of the current unit, and whether one
-  // found the buffer full
+  // exact form: verification requests of the current unit, and whether it
+  // is left to the FP64 band kernel (more than the budget, or the buffer full)
   unsigned unit_reqs;
+  unsigned unit_wide;   // those whose bound exceeds kWideBound
   unsigned unit_lost;
+  unsigned budget, wide_budget;
 };
 
 struct Smem {
@@ -257,6 +263,9 @@ struct Smem {
   long long unit, band, unit_in_band;
   int prob_index;
   SlowCtx cx;
+  // exact form: each warp's block of the request buffer and its used slots
+  unsigned long long rq_base[kWarps];
+  int rq_used[kWarps];
 };
 
 // Filter-table entry: smallest best, largest inverse norm, largest |df|,
@@ -640,61 +649,79 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
   return nreq;
 }
 
-// Exact form, one cell per lane that `cand` marks: its FP32 r lies within
-// its error bound mk of a best.  The bests are read again from the profile
-// keys (the staged copies lag behind the other CTAs); a cell that may still
-// win publishes its lower bound r - mk, so the filters rise at once, and
-// asks for its FP64 r.  Called by the whole warp.
-__device__ __forceinline__ void exact_request(Smem& sm, const SlowCtx& cx, bool cand, float rv,
-                                              float mk, int64_t i, int64_t j, int rslot,
-                                              int cslot, int g, int lane, int& nreq) {
+// Exact form: the unused slots of the warp's block of the request buffer
+// become requests that rule themselves out.
+__device__ __forceinline__ void close_requests(Smem& sm, const SlowCtx& cx, int warp, int lane) {
+  const unsigned long long base = sm.rq_base[warp];
+  for (int s = sm.rq_used[warp] + lane; s < kReqChunk; s += 32)
+    if (base + s < static_cast<unsigned long long>(cx.vcap)) cx.vreq[base + s] = VerifyReq{0, 0, -4.f};
+}
+
+// Exact form: writes the requests of the lanes that qx, qy mark (segments x
+// and y of cells (i, i + d)) into the warp's block of the request buffer,
+// kReqChunk slots taken at a time, so that the global counter's round trip is
+// paid once per block and not once per row of candidates.  Called by the
+// whole warp; returns the number written.
+__device__ __forceinline__ int push_requests(Smem& sm, const SlowCtx& cx, int warp, int lane,
+                                             bool qx, bool qy, float2 rv, float2 mk, int64_t ix,
+                                             int64_t iy, int64_t d) {
+  const unsigned mx = __ballot_sync(0xffffffffu, qx), my = __ballot_sync(0xffffffffu, qy);
+  const int n = __popc(mx) + __popc(my);
+  if (n == 0) return 0;
+  int used = sm.rq_used[warp];
+  unsigned long long base = sm.rq_base[warp];
+  if (used + n > kReqChunk) {
+    close_requests(sm, cx, warp, lane);
+    if (lane == 0) base = atomicAdd(cx.vcount, static_cast<unsigned long long>(kReqChunk));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    used = 0;
+  }
+  const unsigned lt = (1u << lane) - 1u;
+  VerifyReq rq;
+  rq.d = static_cast<uint32_t>(d);
+  const unsigned long long sx = base + used + __popc(mx & lt);
+  const unsigned long long sy = base + used + __popc(mx) + __popc(my & lt);
+  if (qx && sx < static_cast<unsigned long long>(cx.vcap)) {
+    rq.i = static_cast<uint64_t>(ix) | (static_cast<uint64_t>(cx.prob) << 40);
+    rq.ub = rv.x + mk.x;
+    cx.vreq[sx] = rq;
+  }
+  if (qy && sy < static_cast<unsigned long long>(cx.vcap)) {
+    rq.i = static_cast<uint64_t>(iy) | (static_cast<uint64_t>(cx.prob) << 40);
+    rq.ub = rv.y + mk.y;
+    cx.vreq[sy] = rq;
+  }
+  const unsigned wide = __popc(__ballot_sync(0xffffffffu, qx && mk.x > kWideBound)) +
+                        __popc(__ballot_sync(0xffffffffu, qy && mk.y > kWideBound));
+  if (lane == 0) {
+    sm.rq_base[warp] = base;
+    sm.rq_used[warp] = used + n;
+    if (atomicAdd(&sm.cx.unit_reqs, static_cast<unsigned>(n)) + n > cx.budget ||
+        (wide && atomicAdd(&sm.cx.unit_wide, wide) + wide > cx.wide_budget) ||
+        base + used + n > static_cast<unsigned long long>(cx.vcap))
+      sm.cx.unit_lost = 1;
+  }
+  __syncwarp();
+  return n;
+}
+
+// Exact form: a candidate's lower bound lb raises its row's and its column's
+// best at once, in the keys and in the staged copies (which only filter: a
+// racing store of a smaller value costs extra work, never a wrong result).
+__device__ __forceinline__ void publish_bound(Smem& sm, const SlowCtx& cx, float lb, int64_t i,
+                                              int64_t j, int rslot, int cslot, int g) {
   const Problem& pr = *cx.pr;
-  bool open = false;
-  if (cand) {
-    float fr = kNoTarget, fc = kNoTarget;
-    if (pr.key_row) fr = key_corr_floor(__ldcg(pr.key_row + i), cx.kl);
-    if (pr.key_col) fc = key_corr_floor(__ldcg(pr.key_col + j), cx.kl);
-    open = rv + mk > fr || rv + mk > fc;
-    if (open) {
-      const float lb = rv - mk;
-      const uint64_t q = q_from_float_bits(__float_as_uint(lb), cx.kl.frac_bits);
-      if (lb > -2.f && pr.key_row && lb > fr) {
-        atomicMax(reinterpret_cast<u64*>(pr.key_row + i), make_key(q, j, cx.kl));
-        fr = lb;
-      }
-      if (lb > -2.f && pr.key_col && lb > fc) {
-        atomicMax(reinterpret_cast<u64*>(pr.key_col + j), make_key(q, i, cx.kl));
-        fc = lb;
-      }
-    }
-    // the staged copies only filter: a racing store of a smaller value
-    // costs extra work later, never a wrong result
-    float& rb = g ? sm.r_best[rslot].y : sm.r_best[rslot].x;
-    float& cb = g ? sm.c_best[padc(cslot)].y : sm.c_best[padc(cslot)].x;
-    if (fr > rb) rb = fr;
-    if (fc > cb) cb = fc;
+  if (!(lb > -2.f)) return;
+  float& rb = g ? sm.r_best[rslot].y : sm.r_best[rslot].x;
+  float& cb = g ? sm.c_best[padc(cslot)].y : sm.c_best[padc(cslot)].x;
+  const uint64_t q = q_from_float_bits(__float_as_uint(lb), cx.kl.frac_bits);
+  if (lb > rb) {
+    atomicMax(reinterpret_cast<u64*>(pr.key_row + i), make_key(q, j, cx.kl));
+    rb = lb;
   }
-  const unsigned mo = __ballot_sync(0xffffffffu, open);
-  if (!mo) return;
-  const int leader = __ffs(mo) - 1;
-  unsigned long long base = 0;
-  if (lane == leader) {
-    base = atomicAdd(cx.vcount, static_cast<unsigned long long>(__popc(mo)));
-    atomicAdd(&sm.cx.unit_reqs, static_cast<unsigned>(__popc(mo)));
-  }
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (open) {
-    const unsigned long long slot = base + __popc(mo & ((1u << lane) - 1u));
-    ++nreq;
-    if (slot < static_cast<unsigned long long>(cx.vcap)) {
-      VerifyReq rq;
-      rq.i = static_cast<uint64_t>(i) | (static_cast<uint64_t>(cx.prob) << 40);
-      rq.d = static_cast<uint32_t>(j - i);
-      rq.ub = rv + mk;
-      cx.vreq[slot] = rq;
-    } else {
-      sm.cx.unit_lost = 1;  // the FP64 band kernel takes the unit
-    }
+  if (lb > cb) {
+    atomicMax(reinterpret_cast<u64*>(pr.key_col + j), make_key(q, i, cx.kl));
+    cb = lb;
   }
 }
 
@@ -705,6 +732,9 @@ __device__ __forceinline__ void exact_request(Smem& sm, const SlowCtx& cx, bool 
 __device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane) {
   __syncwarp();  // the queue was written by other lanes
   const SlowCtx& cx = sm.cx;
+  // a unit left to the FP64 kernel needs no more requests (lane 0's view:
+  // another warp may be setting it)
+  if (__shfl_sync(0xffffffffu, *const_cast<volatile unsigned*>(&sm.cx.unit_lost), 0)) return 0;
   const int k = lane & 7;
   int nreq = 0;
   for (int p = 0; p < count; p += 4) {
@@ -742,12 +772,13 @@ __device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane)
       const bool cy_ = live && rv.y + mk.y > fminf(rb.y, cbv.y);
       if (!__any_sync(0xffffffffu, cx_ || cy_)) continue;
       const int64_t i0 = cx.rbase[0] + r0 + rr, i1 = cx.rbase[1] + r0 + rr;
-      exact_request(sm, cx, cx_, rv.x, mk.x, i0, i0 + jd, r0 + rr, rcs, 0, lane, nreq);
-      exact_request(sm, cx, cy_, rv.y, mk.y, i1, i1 + jd, r0 + rr, rcs, 1, lane, nreq);
+      nreq += push_requests(sm, cx, warp, lane, cx_, cy_, rv, mk, i0, i1, jd);
+      if (cx_) publish_bound(sm, cx, rv.x - mk.x, i0, i0 + jd, r0 + rr, rcs, 0);
+      if (cy_) publish_bound(sm, cx, rv.y - mk.y, i1, i1 + jd, r0 + rr, rcs, 1);
     }
   }
   __syncwarp();
-  return nreq;
+  return lane == 0 ? nreq : 0;
 }
 
 // Bound on the error of a thread's FP32 anchors (exact form), per segment,
@@ -1002,6 +1033,8 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
   if constexpr (kExact) {
     const float vmax = __uint_as_float(P.range[0]), imax = __uint_as_float(P.range[1]);
     out_of_range = !(vmax <= kExactMaxValue && imax <= kExactMaxInv && vmax * imax <= kExactMaxRatio);
+    if (lane == 0) sm.rq_used[warp] = kReqChunk;  // no block yet
+    __syncwarp();
   }
 
   for (;;) {
@@ -1010,7 +1043,10 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       sm.unit = uu;
       if constexpr (kExact) {
         sm.cx.unit_reqs = 0;
+        sm.cx.unit_wide = 0;
         sm.cx.unit_lost = 0;
+        sm.cx.budget = P.req_budget;
+        sm.cx.wide_budget = P.wide_budget;
         if (!kBound && out_of_range && uu < P.total_units)
           P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = uu;
       }
@@ -1303,6 +1339,12 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
     // ---------------- slabs ----------------
     const int64_t nslabs = (seg_len[0] + kSlab - 1) / kSlab;
     for (int64_t q = 0; q < nslabs; ++q) {
+      // steps with rows of the segment (whole pairs), and the staged columns
+      // that they reach (sums and bounds: later slabs stage every entering
+      // column, which flushes the previous one in its place)
+      const int64_t left = seg_len[0] - q * kSlab;
+      const int nsteps = left >= kSlab ? kSteps : static_cast<int>((left + 15) / 16) * 2;
+      const int ncols = (kSum || kBound) && q > 0 ? kCols : (kBand + nsteps * kRows + 31) / 32 * 32;
       int64_t rbase[2], rend[2], cbase_g[2];
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
@@ -1345,7 +1387,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         }
       }
 #pragma unroll 3
-      for (int c = (q == 0 ? 0 : kCols - kSlab) + t; c < kCols; c += kThreads) {
+      for (int c = (q == 0 ? 0 : kCols - kSlab) + t; c < ncols; c += kThreads) {
         const int rc = ringc(ring0, c);
         const int64_t j0 = cbase_g[0] + c, j1 = cbase_g[1] + c;
         const bool ok0 = seg_len[0] > 0 && j0 < pr.C.ns;
@@ -1869,7 +1911,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         }
       };
 #pragma unroll 1
-      for (int s = 0; s < kSteps; s += 2) {
+      for (int s = 0; s < nsteps; s += 2) {
         {
           const int rb = (rq + s + t) < kBlocks ? (rq + s + t) : (rq + s + t - kBlocks);
           if constexpr (kWindow) {
@@ -1886,7 +1928,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         // between pairs: drain a half-full queue (every queue at the slab's
         // end), then queue and drain the steps that found it full
         const unsigned pmask = __ballot_sync(0xffffffffu, pend >= 0);
-        if (pmask || qn >= kQueue / 2 || (qn && s + 2 == kSteps)) {
+        if (pmask || qn >= kQueue / 2 || (qn && s + 2 == nsteps)) {
           if (qn) {
             n_verify += kExact ? drain_exact(sm, warp, qn, lane)
                                : drain_queue<!kCoarse>(sm, warp, qn, lane);
@@ -1912,7 +1954,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
       if constexpr (kBound) {
         // the columns after the last step's first 8
-        const int rb = (rq + kSteps + t) < kBlocks ? (rq + kSteps + t) : (rq + kSteps + t - kBlocks);
+        const int rb = (rq + nsteps + t) < kBlocks ? (rq + nsteps + t) : (rq + nsteps + t - kBlocks);
 #pragma unroll
         for (int x = 0; x < kDiags - 1; ++x)
           raise_shared(sm.c_best[9 * rb + x], __float_as_uint(cnext[x].x), __float_as_uint(cnext[x].y));
@@ -1921,7 +1963,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         raise_bound(pr.key_row, rbase[0] + t, v.x, P.kl);
         raise_bound(pr.key_row, rbase[1] + t, v.y, P.kl);
         if (q + 1 == nslabs) {
-          for (int c = t; c < kCols; c += kThreads) {
+          for (int c = t; c < ncols; c += kThreads) {
             const float2 u = sm.c_best[padc(ringc(ring0, c))];
             raise_bound(pr.key_col, cbase_g[0] + c, u.x, P.kl);
             raise_bound(pr.key_col, cbase_g[1] + c, u.y, P.kl);
@@ -1930,14 +1972,14 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         }
         continue;
       }
-      n_steps += kSteps;
+      n_steps += nsteps;
       __syncthreads();
       if constexpr (kExact) {
         // A unit whose cells its FP32 values cannot rule out (error bounds
         // above the spread of the correlations: near-flat windows beside
         // large steps, exact repeats everywhere) is left to the FP64 band
         // kernel; what it published stands.
-        const bool leave = sm.cx.unit_reqs > P.req_budget || sm.cx.unit_lost;
+        const bool leave = sm.cx.unit_lost;
         __syncthreads();
         if (leave) {
           if (t == 0) P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = u;
@@ -1953,7 +1995,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
       if (sum_mode && pr.sum_col && q + 1 == nslabs) {
         // unit end: every column left in the ring
-        for (int c = t; c < kCols; c += kThreads) {
+        for (int c = t; c < ncols; c += kThreads) {
           const float2 v = sm.c_best[padc(ringc(ring0, c))];
           const int64_t j0 = cbase_g[0] + c, j1 = cbase_g[1] + c;
           if (v.x != 0.f && j0 < pr.C.ns) atomicAdd(pr.sum_col + j0, static_cast<double>(v.x));
@@ -1964,6 +2006,12 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       // overwrites when it fetches the next unit.
       if (sum_mode && q + 1 == nslabs) __syncthreads();
     }
+  }
+  if constexpr (kExact && !kBound) {
+    __syncwarp();
+    sm.cx.vcap = P.vreq_cap;  // (a CTA without a unit has no context; every writer the same)
+    sm.cx.vreq = P.vreq;
+    close_requests(sm, sm.cx, warp, lane);
   }
   // per-CTA totals of the work counters
 #pragma unroll
