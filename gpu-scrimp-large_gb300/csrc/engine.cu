@@ -159,6 +159,17 @@ constexpr int64_t kWidePerCells = 1024;
 // the direct-dot seeds at 1/32 of the FP64 pipe's work.
 int64_t fp64_segment(int64_t m) { return std::max<int64_t>(32 * m, 8192); }
 
+// Segment length of the FP64 band kernel: fp64_segment, less where the join
+// is small.  As in exact_segment, with 7 m / 4 operations per diagonal for a
+// seed and 4 per cell: v waves of units are best at v = sqrt(8 K_1 / 7 m)
+// (32768 samples, m = 128: 64-row segments, 8 waves, spent three fifths of
+// the FP64 pipe on seeds).
+int64_t fp64_rows(double cells, int64_t resident, int W, int slab, int64_t m) {
+  const double k1 = cells / (2.0 * W * static_cast<double>(resident));
+  const double v = std::min(8.0, std::max(1.5, std::sqrt(8.0 / 7.0 * k1 / static_cast<double>(m))));
+  return std::min(fp64_segment(m), (static_cast<int64_t>(k1 / v) / slab + 1) * slab);
+}
+
 // Bound on |reported r - FP64 r| after final_eval_kernel: twice
 // gamma_{ceil(m/16) + 10} (u = 2^-53) for the direct FP64 evaluation, plus
 // the key's resolution 2^-F (final_eval.cu derives it).
@@ -986,12 +997,14 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   }
   if (kind == K_EXACT) {
     K = std::min(K, exact_segment(cells_d, resident, W, slab, m));
+  } else if (kind == K_FP64) {
+    K = fp64_rows(cells_d, resident, W, slab, m);
   } else {
     K = std::min(K, std::max<int64_t>(k_lb, slab));
     K = std::max<int64_t>(slab, (K / slab) * slab);
   }
-  {
-    // The mixed 1NN kernel pairs the two segments of a unit; their column
+  if (band) {
+    // The FP32 band kernel pairs the two segments of a unit; their column
     // spans must be a whole number of FP32-copy blocks apart.
     const int64_t blk = 1ll << block_shift(m);
     if (K % blk) K = std::max<int64_t>(blk, (K / blk) * blk);
@@ -1911,14 +1924,7 @@ int run_device_noalloc(const NoAllocDevice& dv, const scamp_c_args* a, scamp_c_r
   const int64_t resident = static_cast<int64_t>(dv.sms) * dv.occ;
   // segment length: the FP64 rule of run_device()
   const double cells_d = static_cast<double>(plan.cells);
-  const int64_t k_lb = static_cast<int64_t>(cells_d / (8.0 * resident * 2.0 * W));
-  int64_t K = fp64_segment(m);
-  K = std::min(K, std::max<int64_t>(k_lb, slab));
-  K = std::max<int64_t>(slab, (K / slab) * slab);
-  {
-    const int64_t blk = 1ll << block_shift(m);
-    if (K % blk) K = std::max<int64_t>(blk, (K / blk) * blk);
-  }
+  const int64_t K = fp64_rows(cells_d, resident, W, slab, m);
 
   JoinParams P{};
   // The band prefix is counted here (for the total and the grid) and built

@@ -52,6 +52,31 @@ __device__ __forceinline__ int64_t ord_double(double x) {
   return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll);
 }
 
+// SUM_THRESH adds in fixed point: r as a signed integer in units of 2^-53
+// (the last place of r in [1/2, 1), the bits below cut off), integer pipe
+// only.  Integer sums are exact, so a slab's sum (at most 512 cells, |r| <= 1
+// up to rounding: 2^62) carries less error than one added in FP64, and they
+// leave the FP64 pipe the recurrence's four operations per cell: the two
+// additions per cell and the row reductions' shuffles in FP64 had taken three
+// quarters of the pipe (32768 samples, m = 128, r > 0.9: 14.1 -> 9.7 ms, and 4.8
+// with the segments of fp64_rows(): 88% of the FP64 pipe).  A value beyond
+// 1.5 (a recurrence that lost everything to a spike) counts as 1.5, so that
+// no slab's sum can wrap around.
+constexpr int kSumFrac = 53;
+__device__ __forceinline__ long long fixed_r(double r) {
+  const uint64_t bits = static_cast<uint64_t>(__double_as_longlong(r));
+  const int e = static_cast<int>((bits >> 52) & 0x7FF);
+  const uint64_t sig = (bits & 0x000FFFFFFFFFFFFFull) | (e ? (1ull << 52) : 0);
+  const int s = 1075 - kSumFrac - e;  // |r| 2^53 = sig 2^-s
+  constexpr uint64_t kMost = 3ull << (kSumFrac - 1);
+  uint64_t mag = s >= 64 ? 0 : (s >= 0 ? sig >> s : (s == -1 ? sig << 1 : kMost));
+  if (mag > kMost) mag = kMost;
+  return (bits >> 63) ? -static_cast<long long>(mag) : static_cast<long long>(mag);
+}
+__device__ __forceinline__ double sum_of_fixed(unsigned long long v) {
+  return static_cast<double>(static_cast<long long>(v)) * (1.0 / (1ull << kSumFrac));
+}
+
 struct SmemFp64 {
   double df_r[2][kSlab], dg_r[2][kSlab], iv_r[2][kSlab];
   double df_c[2][kCols], dg_c[2][kCols], iv_c[2][kCols];
@@ -61,8 +86,8 @@ struct SmemFp64 {
       unsigned long long row[2][kSlab];
     } key;
     struct {
-      double col[2][kCols];
-      double row[2][kSlab];
+      unsigned long long col[2][kCols];  // fixed point, two's complement
+      unsigned long long row[2][kSlab];
     } sum;
   } prof;
   unsigned char dirty_col[2][kCols];
@@ -70,24 +95,39 @@ struct SmemFp64 {
   long long unit;
 };
 
-// FP64 direct-dot seed: cov of row window i and column window j, each centred
-// by its own mean (the reference's QT seed, src/qt_helper.cpp:52-72).  Four
-// interleaved accumulators keep the FP64 pipe fed.
-__device__ double seed_fp64(const SeriesDev& R, const SeriesDev& C, int64_t i,
-                            int64_t j, int64_t m) {
+// FP64 direct-dot seeds: the covariances of row window i with the column
+// windows j .. j + kDiags - 1 (the reference's QT seed,
+// src/qt_helper.cpp:52-72).  The row window is centred by its own mean, the
+// column samples by the first window's, which the four windows share:
+//   cov_k = sum x_t y_{t+k} - (mean_{j+k} - mean_j) sum x_t,
+// 7 FP64 operations per sample for four windows against 12 with each window
+// centred by itself.  Windows at or past C.ns get 0.
+__device__ __forceinline__ void seed_fp64(const SeriesDev& R, const SeriesDev& C, int64_t i,
+                                          int64_t j, int64_t m, double (&cov)[kDiags]) {
+#pragma unroll
+  for (int k = 0; k < kDiags; ++k) cov[k] = 0.0;
+  if (j >= C.ns) return;
   const double mr = R.mean[i], mc = C.mean[j];
   const double* __restrict__ tr = R.T + i;
   const double* __restrict__ tc = C.T + j;
-  double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-  int64_t t = 0;
-  for (; t + 4 <= m; t += 4) {
-    a0 = fma(tr[t] - mr, tc[t] - mc, a0);
-    a1 = fma(tr[t + 1] - mr, tc[t + 1] - mc, a1);
-    a2 = fma(tr[t + 2] - mr, tc[t + 2] - mc, a2);
-    a3 = fma(tr[t + 3] - mr, tc[t + 3] - mc, a3);
+  const int64_t nc = C.n - j;  // column samples from j on
+  double xs = 0.0;
+  double y[kDiags];
+#pragma unroll
+  for (int k = 0; k + 1 < kDiags; ++k) y[k] = k < nc ? tc[k] - mc : 0.0;
+#pragma unroll 4
+  for (int64_t t = 0; t < m; ++t) {
+    const double x = tr[t] - mr;
+    y[kDiags - 1] = t + kDiags - 1 < nc ? tc[t + kDiags - 1] - mc : 0.0;
+    xs += x;
+#pragma unroll
+    for (int k = 0; k < kDiags; ++k) cov[k] = fma(x, y[k], cov[k]);
+#pragma unroll
+    for (int k = 0; k + 1 < kDiags; ++k) y[k] = y[k + 1];
   }
-  for (; t < m; ++t) a0 = fma(tr[t] - mr, tc[t] - mc, a0);
-  return (a0 + a1) + (a2 + a3);
+#pragma unroll
+  for (int k = 0; k < kDiags; ++k)
+    cov[k] = j + k < C.ns ? fma(-(C.mean[j + k] - mc), xs, cov[k]) : 0.0;
 }
 
 }  // namespace
@@ -145,13 +185,13 @@ join_fp64_kernel(JoinParams P) {
 
     // Seeds for this thread's diagonals.
     double cov[2][kDiags];
+#pragma unroll
     for (int g = 0; g < 2; ++g) {
-      for (int k = 0; k < kDiags; ++k) {
-        const int64_t d = d_my + k;
-        const int64_t i = seg_row[g];
-        cov[g][k] = 0;
-        if (seg_len[g] > 0 && d < pr.d_hi && i + d < pr.C.ns)
-          cov[g][k] = seed_fp64(pr.R, pr.C, i, i + d, P.m);
+      if (seg_len[g] > 0) {
+        seed_fp64(pr.R, pr.C, seg_row[g], seg_row[g] + d_my, P.m, cov[g]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kDiags; ++k) cov[g][k] = 0.0;
       }
     }
     // Per-diagonal validity (diagonal range and the is_aligned exclusion).
@@ -176,7 +216,7 @@ join_fp64_kernel(JoinParams P) {
           if (is_1nn) {
             sm.prof.key.row[g][x] = (ok && pr.key_row) ? pr.key_row[i] : 0ull;
           } else {
-            sm.prof.sum.row[g][x] = 0.0;
+            sm.prof.sum.row[g][x] = 0ull;
           }
           sm.dirty_row[g][x] = 0;
         }
@@ -190,7 +230,7 @@ join_fp64_kernel(JoinParams P) {
           if (is_1nn) {
             sm.prof.key.col[g][x] = (ok && pr.key_col) ? pr.key_col[j] : 0ull;
           } else {
-            sm.prof.sum.col[g][x] = 0.0;
+            sm.prof.sum.col[g][x] = 0ull;
           }
           sm.dirty_col[g][x] = 0;
         }
@@ -270,8 +310,8 @@ join_fp64_kernel(JoinParams P) {
           }
         } else {
           // SUM_THRESH: sum r over cells with r > threshold.
-          double csum[2][kDiags + kRows - 1];
-          double rsum[2][kRows];
+          unsigned long long csum[2][kDiags + kRows - 1];
+          unsigned long long rsum[2][kRows];
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
 #pragma unroll
@@ -291,10 +331,10 @@ join_fp64_kernel(JoinParams P) {
                 const int c = cb + rr + k;
                 const double r = fmul_dfma(fmul_dfma(cov[g][k], sm.iv_c[g][c]), ivr);
                 const bool take = dvalid[k] && ord_double(r) > ord_thr;
-                if (take) {
-                  rsum[g][rr] += r;
-                  csum[g][rr + k] += r;
-                }
+                const unsigned long long v =
+                    take ? static_cast<unsigned long long>(fixed_r(r)) : 0ull;
+                rsum[g][rr] += v;
+                csum[g][rr + k] += v;
                 cov[g][k] = fma(sm.df_c[g][c], dgr, cov[g][k]);
                 cov[g][k] = fma(dfr, sm.dg_c[g][c], cov[g][k]);
               }
@@ -305,17 +345,17 @@ join_fp64_kernel(JoinParams P) {
             for (int g = 0; g < 2; ++g)
 #pragma unroll
               for (int c = 0; c < kDiags + kRows - 1; ++c)
-                if (csum[g][c] != 0.0) atomicAdd(&sm.prof.sum.col[g][cb + c], csum[g][c]);
+                if (csum[g][c] != 0) atomicAdd(&sm.prof.sum.col[g][cb + c], csum[g][c]);
           }
           if (pr.sum_row) {
 #pragma unroll
             for (int g = 0; g < 2; ++g)
 #pragma unroll
               for (int rr = 0; rr < kRows; ++rr) {
-                double v = rsum[g][rr];
+                unsigned long long v = rsum[g][rr];
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == 0 && v != 0.0) atomicAdd(&sm.prof.sum.row[g][r0 + rr], v);
+                if (lane == 0 && v != 0) atomicAdd(&sm.prof.sum.row[g][r0 + rr], v);
               }
           }
         }
@@ -341,12 +381,12 @@ join_fp64_kernel(JoinParams P) {
         } else {
           if (pr.sum_col)
             for (int x = t; x < kCols; x += kThreads) {
-              const double v = sm.prof.sum.col[g][x];
+              const double v = sum_of_fixed(sm.prof.sum.col[g][x]);
               if (v != 0.0 && cbase + x < pr.C.ns) atomicAdd(&pr.sum_col[cbase + x], v);
             }
           if (pr.sum_row)
             for (int x = t; x < kSlab; x += kThreads) {
-              const double v = sm.prof.sum.row[g][x];
+              const double v = sum_of_fixed(sm.prof.sum.row[g][x]);
               if (v != 0.0 && rbase + x < rend) atomicAdd(&pr.sum_row[rbase + x], v);
             }
         }
