@@ -219,10 +219,23 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
     }
     // Sums of squares: the recurrence's terms with the means' low parts, so
     // that a large offset's rounded mean does not leave a per-step residue
-    // (b - a)(delta_w + delta_w+1).
+    // (b - a)(delta_w + delta_w+1).  Each term is a compensated product: one
+    // rounding of a spike's term would stay in every later sum of the chunk
+    // (2^-53 of the spike's square, 1e-6 of the norm behind a spike of 10^6
+    // standard deviations).
     double es = 0, ec = 0;
-    if (active && has_next)
-      es = (((x_out - mu) - mu_lo) + ((x_in - mu_next) - mu_next_lo)) * (x_in - x_out);
+    if (active && has_next) {
+      double ph = 0, pl = 0, qh = 0, ql = 0;
+      acc2(ph, pl, x_out);
+      acc2(ph, pl, -mu);
+      acc2(ph, pl, x_in);
+      acc2(ph, pl, -mu_next);
+      pl -= mu_lo + mu_next_lo;
+      acc2(qh, ql, x_in);
+      acc2(qh, ql, -x_out);
+      es = ph * qh;
+      ec = fma(ph, qh, -es) + fma(ph, ql, pl * qh);
+    }
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
       const double us = __shfl_up_sync(kAll, es, s), uc = __shfl_up_sync(kAll, ec, s);
