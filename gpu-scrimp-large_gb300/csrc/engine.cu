@@ -353,7 +353,7 @@ struct Workspace {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t evk0 = nullptr, evk1 = nullptr;  // around the join kernels
   cudaEvent_t evkv = nullptr;                   // before the verification kernel
-  int fp64_occ = 1;                             // resident join_fp64_kernel CTAs per SM
+  int fp64_occ = 1, visit_occ = 1;  // resident CTAs per SM of the FP64 and visit kernels
   bool timed_kernel = false;
   bool timed_verify = false;
   // the mixed form's largest trusted drift margin (work counter 4) is the
@@ -434,6 +434,7 @@ enum Slot {
   S_BHI_B, S_BLO_B, S_MUREL_B, S_VREQ, S_PAA_A, S_PAA_B, S_SEED_A, S_SEED_B,
   S_BATCH, S_MAX_A, S_MAX_B, S_KNN_A, S_KNN_B, S_MAT,
   S_TC_TAB, S_TC_W, S_TC_XS, S_TC_RAW, S_TC_OUT, S_TC_XI, S_FP64_LIST,
+  S_FP64_UNIT, S_KNN_BOUND_A, S_KNN_BOUND_B, S_MAT_BOUND,
 };
 
 #define CUDA_TRY(expr)                                                     \
@@ -505,14 +506,25 @@ void launch_stats(const double* raw, int64_t n, int64_t m, bool ultra, const Ser
   stats_kernel<<<static_cast<unsigned>(stats_blocks(n - m + 1)), kStatsThreads, 0, st>>>(j, ultra ? 1 : 0);
 }
 
+// Makes `keys` the target of side s (0 = A, 1 = B) in every problem of P.
+void set_keys(JoinParams& P, const Plan& plan, int s, uint64_t* keys) {
+  for (int p = 0; p < P.nprob; ++p) {
+    if (plan.probs[p].col_target == s) P.prob[p].key_col = keys;
+    if (plan.probs[p].row_target == s) P.prob[p].key_row = keys;
+  }
+}
+
 // The bounds pass over the units of P (its own queue head).
 int launch_bounds(const JoinParams& P, bool exact, int64_t grid, size_t smem, cudaStream_t st,
                   std::string* msg) {
-  const void* fn = exact ? reinterpret_cast<const void*>(bound_exact_1nn_kernel)
+  const void* fn = P.mat ? reinterpret_cast<const void*>(bound_exact_mat_kernel)
+                 : exact ? reinterpret_cast<const void*>(bound_exact_1nn_kernel)
                          : reinterpret_cast<const void*>(bound_mixed_1nn_kernel);
   CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem)));
-  if (exact)
+  if (P.mat)
+    bound_exact_mat_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
+  else if (exact)
     bound_exact_1nn_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
   else
     bound_mixed_1nn_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
@@ -777,7 +789,22 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   const bool is_knn = a->profile_type == SCAMP_PROFILE_APPROX_ALL_NEIGHBORS;
   const bool knn_mixed = is_knn && mixed && a->max_matches_per_column >= 1 &&
                          a->max_matches_per_column <= knn_mixed_max_k();
-  const bool visit = (is_knn && !knn_mixed) || (is_mat && !mat_mixed);
+  // Both in double: the exact form (the FP32 band kernel with deterministic
+  // bounds, every cell not ruled out in FP64), the matrix under the mixed
+  // form's condition, the lists where each window sees bands enough for a
+  // bound of its k-th best (2 k of them); else the visit kernel.  20011
+  // samples, m = 128, k = 5 above 0.5: visit kernel 6.3 ms; 30000 samples, m =
+  // 100, 50 x 50 entries: 6.9 ms.
+  const bool fp64_exact = a->precision_type == SCAMP_PRECISION_DOUBLE && !nested &&
+                          plan.m <= kExactMaxWindow;
+  const bool mat_exact = is_mat && fp64_exact && mat_rpc >= kMatMixedMinSpan &&
+                         mat_cpc >= kMatMixedMinSpan &&
+                         std::max(plan.ns_a, plan.ns_b) < (int64_t{1} << 31) &&
+                         static_cast<int64_t>(a->matrix_height) * a->matrix_width < (int64_t{1} << 31);
+  const bool knn_exact = is_knn && fp64_exact && a->max_matches_per_column <= knn_mixed_max_k() &&
+                         std::min(plan.ns_a, plan.ns_b) >=
+                             int64_t{2} * mixed_1nn_band_width() * a->max_matches_per_column;
+  const bool visit = (is_knn && !knn_mixed && !knn_exact) || (is_mat && !mat_mixed && !mat_exact);
   const bool ultra = a->precision_type == SCAMP_PRECISION_ULTRA;
   const int64_t m = plan.m;
   const int64_t na = static_cast<int64_t>(a->len_a);
@@ -799,8 +826,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
 
   // FP64 1NN joins on the mixed band kernel: cells that deterministic bounds
   // cannot rule out get their FP64 r, so the profile is the FP64 one
-  const bool exact = is_1nn && a->precision_type == SCAMP_PRECISION_DOUBLE && !nested &&
-                     m <= kExactMaxWindow;
+  const bool exact = (is_1nn && fp64_exact) || mat_exact || knn_exact;
 
   // ---- seeds: block-averaged pre-pass (mixed 1NN joins that pay for it) ----
   NvtxRange nvtx_join(nested ? "seeding pre-pass join" : "join");
@@ -961,6 +987,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                        (a->filter_mode == 0 && is_1nn && m >= kCoarseFilterMinWindow));
   const void* kfn = kind == K_VISIT ? reinterpret_cast<const void*>(join_visit_kernel)
                   : kind == K_FP64 ? reinterpret_cast<const void*>(join_fp64_kernel)
+                  : mat_exact ? reinterpret_cast<const void*>(join_exact_mat_kernel)
                   : kind == K_EXACT ? reinterpret_cast<const void*>(join_exact_1nn_kernel)
                   : is_mat ? reinterpret_cast<const void*>(join_mixed_mat_kernel)
                   : is_knn ? reinterpret_cast<const void*>(join_mixed_knn_kernel)
@@ -1057,9 +1084,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   P.knn_k = knn_mixed ? static_cast<int>(knn_k) : 0;
   P.threshold = a->distance_threshold;
   P.kl = kl;
-  if (mat_mixed) {
+  if (mat_mixed || mat_exact) {
     P.mat = vmat;
     P.mat_w = a->matrix_width;
+    P.mat_h = a->matrix_height;
     P.rows_per_cell = mat_rpc;
     P.cols_per_cell = mat_cpc;
     // ceil(2^64 / d) for d >= 2
@@ -1106,9 +1134,15 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       void* q;
       if ((rc = ensure(ws, S_FP64_LIST, static_cast<size_t>(P.total_units) * 8, &q, msg))) return rc;
       P.fp64_list = static_cast<int64_t*>(q);
+      if ((rc = ensure(ws, S_FP64_UNIT, static_cast<size_t>(P.total_units), &q, msg))) return rc;
+      P.fp64_unit = static_cast<unsigned char*>(q);
+      CUDA_TRY(cudaMemsetAsync(q, 0, static_cast<size_t>(P.total_units), st));
       P.fp64_count = dcount + 8;
       P.range = range;
-      P.req_budget = static_cast<unsigned>(2 * K * W / kReqPerCells);
+      // (lists: their k-th bests rise too late to rule many out, so no more
+      // than cost half of what the unit costs the visit kernel)
+      P.req_budget = static_cast<unsigned>(is_knn ? 2 * K * W * 2 / std::max<int64_t>(m, 8)
+                                                  : 2 * K * W / kReqPerCells);
       P.wide_budget = static_cast<unsigned>(2 * K * W / kWidePerCells);
     }
     if (band) {
@@ -1133,12 +1167,58 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       ws.timed_kernel = true;
     }
     // ---- bounds pass: joins without seeds start from lower bounds ----
-    if ((kind == K_EXACT || (kind == K_MIXED && is_1nn)) && !seed_a && !use_tc) {
+    if (mat_exact) {
+      // of every grid entry, in a grid of their own
+      void* q;
+      if ((rc = ensure(ws, S_MAT_BOUND, mat_n * 4, &q, msg))) return rc;
+      CUDA_TRY(cudaMemsetAsync(q, 0, mat_n * 4, st));
+      P.mat = static_cast<unsigned*>(q);
+    } else if (knn_exact) {
+      // of every window's k best, in lists of their own
+      for (int s = 0; s < 2; ++s) {
+        if (!vkeys[s]) continue;
+        void* q;
+        if ((rc = ensure(ws, s ? S_KNN_BOUND_B : S_KNN_BOUND_A, nsz[s] * knn_k * 8, &q, msg))) return rc;
+        CUDA_TRY(cudaMemsetAsync(q, 0, nsz[s] * knn_k * 8, st));
+        set_keys(P, plan, s, static_cast<uint64_t*>(q));
+      }
+      P.knn_k = static_cast<int>(knn_k);
+    }
+    if (exact || (kind == K_MIXED && is_1nn && !seed_a && !use_tc)) {
       JoinParams B = P;
       B.unit_counter = dcount + 11;
       if ((rc = launch_bounds(B, exact, grid, smem, st, msg))) return rc;
       ++launches;
     }
+    if (knn_exact) {
+      for (int s = 0; s < 2; ++s) {
+        if (!vkeys[s]) continue;
+        void *q, *bounds = ws.bufs[s ? S_KNN_BOUND_B : S_KNN_BOUND_A].p;
+        if ((rc = ensure(ws, s ? S_KEY_B : S_KEY_A, nsz[s] * 8, &q, msg))) return rc;
+        knn_floor_kernel<<<static_cast<unsigned>((nsz[s] + 255) / 256), 256, 0, st>>>(
+            static_cast<unsigned long long*>(bounds), vkeys[s], nsz[s], static_cast<int>(knn_k),
+            a->distance_threshold, kl, static_cast<uint64_t*>(q));
+        ++launches;
+        set_keys(P, plan, s, static_cast<uint64_t*>(q));
+      }
+    }
+    auto visit_args = [&]() {
+      VisitArgs V{};
+      V.mode = a->profile_type == SCAMP_PROFILE_APPROX_ALL_NEIGHBORS ? 0 : 1;
+      V.topk[0] = vkeys[0];
+      V.topk[1] = vkeys[1];
+      V.k = static_cast<int>(knn_k);
+      V.mat = vmat;
+      V.mat_w = a->matrix_width;
+      // grid rows: windows of B (of A in a self-join), columns: windows of A
+      V.rows_per_cell = V.mode == 1 ? (nsz[1] + a->matrix_height - 1) / a->matrix_height : 1;
+      V.cols_per_cell = V.mode == 1 ? (nsz[0] + a->matrix_width - 1) / a->matrix_width : 1;
+      for (int p = 0; p < P.nprob; ++p) {
+        V.col_target[p] = plan.probs[p].col_target;
+        V.row_target[p] = plan.probs[p].row_target;
+      }
+      return V;
+    };
     auto launch_band = [&](const JoinParams& Q, int64_t g) {
       if (is_mat)
         join_mixed_mat_kernel<<<static_cast<unsigned>(g), nthreads, smem, st>>>(Q);
@@ -1239,34 +1319,31 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
         ++launches;
       }
     } else if (kind == K_EXACT) {
-      join_exact_1nn_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
+      if (mat_exact)
+        join_exact_mat_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
+      else
+        join_exact_1nn_kernel<<<static_cast<unsigned>(grid), nthreads, smem, st>>>(P);
       ++launches;
       if (!nested) {
         CUDA_TRY(cudaEventRecord(ws.evkv, st));
         ws.timed_verify = true;
       }
-      // the units left to FP64 (none in most joins), then the requests
+      // the units left to FP64 (none in most joins), then the requests, both
+      // into the results themselves
       JoinParams F = P;
       F.unit_counter = dcount + 9;
-      join_fp64_kernel<<<static_cast<unsigned>(ws.sms * ws.fp64_occ), fp64_threads(), 0, st>>>(F);
-      verify_exact_kernel<<<static_cast<unsigned>(ws.sms * 8), 256, 0, st>>>(P);
+      F.mat = vmat;
+      for (int s = 0; s < 2 && knn_exact; ++s)
+        if (vkeys[s]) set_keys(F, plan, s, reinterpret_cast<uint64_t*>(vkeys[s]));
+      if (is_1nn)
+        join_fp64_kernel<<<static_cast<unsigned>(ws.sms * ws.fp64_occ), fp64_threads(), 0, st>>>(F);
+      else
+        join_visit_kernel<<<static_cast<unsigned>(ws.sms * ws.visit_occ), visit_threads(), 0, st>>>(
+            F, visit_args());
+      verify_exact_kernel<<<static_cast<unsigned>(ws.sms * 8), 256, 0, st>>>(F);
       launches += 2;
     } else if (kind == K_VISIT) {
-      VisitArgs V{};
-      V.mode = a->profile_type == SCAMP_PROFILE_APPROX_ALL_NEIGHBORS ? 0 : 1;
-      V.topk[0] = vkeys[0];
-      V.topk[1] = vkeys[1];
-      V.k = static_cast<int>(knn_k);
-      V.mat = vmat;
-      V.mat_w = a->matrix_width;
-      // grid rows: windows of B (of A in a self-join), columns: windows of A
-      V.rows_per_cell = V.mode == 1 ? (nsz[1] + a->matrix_height - 1) / a->matrix_height : 1;
-      V.cols_per_cell = V.mode == 1 ? (nsz[0] + a->matrix_width - 1) / a->matrix_width : 1;
-      for (int p = 0; p < P.nprob; ++p) {
-        V.col_target[p] = plan.probs[p].col_target;
-        V.row_target[p] = plan.probs[p].row_target;
-      }
-      join_visit_kernel<<<static_cast<unsigned>(grid), nthreads, 0, st>>>(P, V);
+      join_visit_kernel<<<static_cast<unsigned>(grid), nthreads, 0, st>>>(P, visit_args());
       ++launches;
     } else {
       join_fp64_kernel<<<static_cast<unsigned>(grid), nthreads, 0, st>>>(P);
@@ -1428,7 +1505,10 @@ int init_workspace(int device, Workspace** out, std::string* msg) {
     CUDA_TRY(cudaEventCreate(&ws.evkv));
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &ws.fp64_occ, reinterpret_cast<const void*>(join_fp64_kernel), fp64_threads(), 0));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &ws.visit_occ, reinterpret_cast<const void*>(join_visit_kernel), visit_threads(), 0));
     ws.fp64_occ = std::max(ws.fp64_occ, 1);
+    ws.visit_occ = std::max(ws.visit_occ, 1);
     ws.device = device;
   }
   *out = &ws;

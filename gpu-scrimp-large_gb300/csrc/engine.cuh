@@ -87,6 +87,32 @@ __device__ __forceinline__ float key_corr_floor(uint64_t key, const KeyLayout& k
   return v - 2.0f;                                          // exact for v in [1, 4)
 }
 
+// Inserts `key` into a list of k keys kept largest first: each slot keeps
+// the larger of its key and the incoming one and passes the smaller on, so
+// after every insertion slot s holds the (s+1)-th largest key inserted.
+__device__ __forceinline__ void topk_insert(unsigned long long* slots, int k,
+                                            unsigned long long key) {
+  for (int s = 0; s < k && key != 0; ++s) {
+    const unsigned long long old = atomicMax(slots + s, key);
+    if (old < key) key = old;  // the displaced key moves on
+  }
+}
+
+// Order-preserving uint32 image of a float (not NaN), and back.
+__device__ __forceinline__ unsigned ord_float(float x) {
+  const unsigned b = __float_as_uint(x);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float float_of_ord(unsigned b) {
+  return __uint_as_float((b & 0x80000000u) ? (b & 0x7FFFFFFFu) : ~b);
+}
+
+// n / d for n < 2^32 and d >= 2 from M = ceil(2^64 / d): exact while
+// n d < 2^64 (floor(n M / 2^64) = n / d + n e / (d 2^64), e = M d - 2^64 < d).
+__device__ __forceinline__ int64_t div_magic(int64_t n, uint64_t M) {
+  return static_cast<int64_t>(__umul64hi(static_cast<uint64_t>(n), M));
+}
+
 // ---------------------------------------------------------------------------
 // Series statistics resident in HBM (one set per input series).
 // ---------------------------------------------------------------------------
@@ -183,11 +209,13 @@ struct JoinParams {
   // with their division magics ceil(2^64 / d), and per problem whether its
   // column results (cell (i, j) -> grid (i / rpc, j / cpc)) and its row
   // results (-> grid (j / rpc, i / cpc)) enter the grid.
-  // APPROX_ALL_NEIGHBORS, mixed form: k > 0 makes key_row / key_col lists
-  // of k keys per window (largest first) instead of one key
+  // APPROX_ALL_NEIGHBORS: k > 0 makes key_row / key_col lists of k keys per
+  // window (largest first) instead of one key (exact form: in its bounds
+  // pass and its verification; the join between them reads one key per
+  // window, the bound of its k-th best, and raises none)
   int knn_k;
   unsigned* mat;
-  int64_t mat_w;
+  int64_t mat_w, mat_h;
   int64_t rows_per_cell, cols_per_cell;
   uint64_t rpc_magic, cpc_magic;
   int mat_col[kMaxProblems], mat_row[kMaxProblems];
@@ -199,6 +227,7 @@ struct JoinParams {
   const unsigned* range;
   int64_t* fp64_list;
   unsigned long long* fp64_count;
+  unsigned char* fp64_unit;  // per unit: 1 = left (its requests are void)
   unsigned req_budget, wide_budget;  // all of them, those of wide bounds
 };
 
@@ -305,11 +334,18 @@ __global__ void join_mixed_1nn_coarse_kernel(JoinParams P);
 __global__ void join_mixed_sum_coarse_kernel(JoinParams P);
 __global__ void join_mixed_mat_kernel(JoinParams P);  // mixed MATRIX_SUMMARY
 __global__ void join_mixed_knn_kernel(JoinParams P);  // mixed APPROX_ALL_NEIGHBORS
-__global__ void join_exact_1nn_kernel(JoinParams P);  // FP64 1NN behind the FP32 filter
+__global__ void join_exact_1nn_kernel(JoinParams P);  // FP64 1NN, k-best behind the FP32 filter
+__global__ void join_exact_mat_kernel(JoinParams P);  // FP64 MATRIX_SUMMARY behind it
 __global__ void verify_exact_kernel(JoinParams P);
 // Lower bounds of every window's best before the join itself (FP64 / mixed)
 __global__ void bound_exact_1nn_kernel(JoinParams P);
 __global__ void bound_mixed_1nn_kernel(JoinParams P);
+__global__ void bound_exact_mat_kernel(JoinParams P);  // of every grid entry
+// Per window, the key of the bound of its k-th best: the largest of the
+// threshold, the bounds list's k-th and the given list's k-th.
+__global__ void knn_floor_kernel(const unsigned long long* __restrict__ bounds,
+                                 const unsigned long long* __restrict__ lists, int64_t n, int k,
+                                 double thr, KeyLayout kl, uint64_t* __restrict__ out);
 __global__ void verify_requests_kernel(JoinParams P);
 
 // Tensor-core anchors of one problem's chunk of anchor rows (anchor_tc.cu).

@@ -204,10 +204,12 @@ __global__ void __launch_bounds__(256) knn_final_eval_kernel(EvalSide S, int k, 
   }
 }
 
-// Settles the exact form's requests: every cell that may be its row's or its
-// column's best gets its FP64 r and competes with it.  A request whose upper
-// bound has meanwhile fallen to or below both bests is skipped (decided by
-// the group's first lane: the lanes' loads of a key need not agree).
+// Settles the exact form's requests: every cell that may count gets its FP64
+// r and enters its row's and its column's results: the best (1NN), the k-best
+// lists (knn_k > 0) or the grid (mat).  A request whose upper bound the
+// results have meanwhile reached is skipped (decided by the group's first
+// lane: the lanes' loads need not agree), and so is one of a unit left to the
+// FP64 kernels, which have entered its cells (a list would hold them twice).
 __global__ void __launch_bounds__(256) verify_exact_kernel(JoinParams P) {
   const int lane = threadIdx.x & 31;
   const int sub = lane & (kLanes - 1);
@@ -216,20 +218,53 @@ __global__ void __launch_bounds__(256) verify_exact_kernel(JoinParams P) {
                         ? static_cast<int64_t>(total) : P.vreq_cap;
   const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
   constexpr int kGroups = 32 / kLanes;
+  const int k = P.knn_k;
+  const bool plain = k == 0 && !P.mat;
+  const bool some_left = *P.fp64_count > 0;
+  const float thr = plain ? -3.f : __double2float_rd(P.threshold);
   for (int64_t g0 = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups;
        g0 < n; g0 += nwarps * kGroups) {
     const int64_t g = g0 + lane / kLanes;
     const VerifyReq rq = P.vreq[g < n ? g : g0];
-    const Problem& pr = P.prob[static_cast<int>(rq.i >> 40)];
+    const int p = static_cast<int>(rq.i >> 40);
+    const Problem& pr = P.prob[p];
     const int64_t i = static_cast<int64_t>(rq.i & ((uint64_t{1} << 40) - 1));
     const int64_t j = i + rq.d;
-    bool row = g < n && pr.key_row && rq.ub > key_corr_floor(__ldcg(pr.key_row + i), P.kl);
-    bool col = g < n && pr.key_col && rq.ub > key_corr_floor(__ldcg(pr.key_col + j), P.kl);
+    bool row, col;
+    unsigned *er = nullptr, *ec = nullptr;  // the cell's grid entries
+    if (P.mat) {
+      if (P.mat_col[p]) ec = P.mat + div_magic(i, P.rpc_magic) * P.mat_w + div_magic(j, P.cpc_magic);
+      if (P.mat_row[p]) er = P.mat + div_magic(j, P.rpc_magic) * P.mat_w + div_magic(i, P.cpc_magic);
+      // (>=: an entry rounded to a float may lie above its FP64 value)
+      row = er && rq.ub >= float_of_ord(__ldcg(er));
+      col = ec && rq.ub >= float_of_ord(__ldcg(ec));
+    } else {
+      row = pr.key_row && rq.ub > key_corr_floor(__ldcg(pr.key_row + (k ? i * k + k - 1 : i)), P.kl);
+      col = pr.key_col && rq.ub > key_corr_floor(__ldcg(pr.key_col + (k ? j * k + k - 1 : j)), P.kl);
+    }
+    bool counts = g < n && rq.ub > thr;
+    if (some_left && counts) {
+      const int64_t band = (static_cast<int64_t>(rq.d) - pr.d_lo) / P.band_width;
+      counts = !P.fp64_unit[P.band_unit_prefix[pr.band_begin + band] + i / (2 * P.seg_len)];
+    }
+    row = row && counts;
+    col = col && counts;
     const unsigned open = __ballot_sync(0xffffffffu, sub == 0 && (row || col));
     if (!open) continue;
     const bool work = (open >> (lane & ~(kLanes - 1))) & 1u;
     const double r = corr_group_norms(pr.R, pr.C, i, j, work ? P.m : 0, sub);
-    if (sub == 0 && work && !isnan(r)) {
+    if (sub != 0 || !work || isnan(r) || !(plain || r > P.threshold)) continue;
+    if (P.mat) {
+      const unsigned v = ord_float(static_cast<float>(r));
+      if (row) atomicMax(er, v);
+      if (col) atomicMax(ec, v);
+    } else if (k) {
+      unsigned long long* lr = reinterpret_cast<unsigned long long*>(pr.key_row + i * k);
+      unsigned long long* lc = reinterpret_cast<unsigned long long*>(pr.key_col + j * k);
+      const uint64_t kr = corr_key(r, j, P.kl), kc = corr_key(r, i, P.kl);
+      if (row && kr > __ldcg(lr + k - 1)) topk_insert(lr, k, kr);
+      if (col && kc > __ldcg(lc + k - 1)) topk_insert(lc, k, kc);
+    } else {
       if (row) atomicMax(reinterpret_cast<unsigned long long*>(pr.key_row + i), corr_key(r, j, P.kl));
       if (col) atomicMax(reinterpret_cast<unsigned long long*>(pr.key_col + j), corr_key(r, i, P.kl));
     }

@@ -215,7 +215,7 @@ struct SlowCtx {
   // problem's targets
   int knn_k;  // APPROX_ALL_NEIGHBORS: list length (0 otherwise)
   unsigned* mat;
-  int64_t mat_w;
+  int64_t mat_w, mat_h;
   int64_t rpc, cpc;
   uint64_t rpc_magic, cpc_magic;
   bool mcol, mrow;
@@ -432,16 +432,6 @@ __device__ __forceinline__ void publish(Smem& sm, const SlowCtx& cx, float rv, i
     atomicMax(reinterpret_cast<u64*>(pr.key_col + j),
               make_key(q_from_float_bits(__float_as_uint(rv), cx.kl.frac_bits), i, cx.kl));
     if (g) sm.c_best[padc(cslot)].y = rv; else sm.c_best[padc(cslot)].x = rv;
-  }
-}
-
-// Inserts `key` into a list of k keys kept largest first: each slot keeps
-// the larger of its key and the incoming one and passes the smaller on, so
-// after every insertion slot s holds the (s+1)-th largest key inserted.
-__device__ __forceinline__ void topk_insert(u64* slots, int k, u64 key) {
-  for (int s = 0; s < k && key != 0; ++s) {
-    const u64 old = atomicMax(slots + s, key);
-    if (old < key) key = old;
   }
 }
 
@@ -725,10 +715,33 @@ __device__ __forceinline__ void publish_bound(Smem& sm, const SlowCtx& cx, float
   }
 }
 
+// Exact matrix form: the smallest bound of the grid entries that the windows
+// a .. a + da (grid rows) and b .. b + db (grid columns) fall in; the spans are
+// shorter than an entry's, so that is two entries each way at most.
+__device__ __forceinline__ float mat_block_floor(const SlowCtx& cx, int64_t a, int64_t da,
+                                                 int64_t b, int64_t db) {
+  const int64_t qa = div_magic(a, cx.rpc_magic), qb = div_magic(b, cx.cpc_magic);
+  const bool ra = a - qa * cx.rpc + da >= cx.rpc && qa + 1 < cx.mat_h;
+  const bool rb = b - qb * cx.cpc + db >= cx.cpc && qb + 1 < cx.mat_w;
+  const unsigned* e = cx.mat + qa * cx.mat_w + qb;
+  unsigned lo = e[0];
+  if (ra) lo = min(lo, e[cx.mat_w]);
+  if (rb) lo = min(lo, e[1]);
+  if (ra && rb) lo = min(lo, e[cx.mat_w + 1]);
+  return lo ? float_of_ord(lo) : -3.f;
+}
+__device__ __forceinline__ float mat_cell_floor(const SlowCtx& cx, int64_t i, int64_t j) {
+  float lo = kNoTarget;
+  if (cx.mcol) lo = mat_block_floor(cx, i, 0, j, 0);
+  if (cx.mrow) lo = fminf(lo, mat_block_floor(cx, j, 0, i, 0));
+  return lo;
+}
+
 // drain_queue() of the exact form: the same walk (rows last to first, the
 // covariance stepped back over each row), with the deterministic bound.  An
 // item's vw is E at the block's end plus the block's own roundings again,
 // for the steps back.
+template <bool kMat>
 __device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane) {
   __syncwarp();  // the queue was written by other lanes
   const SlowCtx& cx = sm.cx;
@@ -765,14 +778,24 @@ __device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane)
       const float2 rv = mul2(mul2(c, ivc), ivr);
       const float2 mk0 = mul2(mul2(vw, ivc), ivr);
       const float2 mk = make_float2(mk0.x + kAbsSlack, mk0.y + kAbsSlack);
-      const float2 rb = sm.r_best[r0 + rr];
-      const float2 cbv = sm.c_best[padc(rcs)];
-      // (false for NaN: excluded diagonals, windows that cannot match)
-      const bool cx_ = live && rv.x + mk.x > fminf(rb.x, cbv.x);
-      const bool cy_ = live && rv.y + mk.y > fminf(rb.y, cbv.y);
-      if (!__any_sync(0xffffffffu, cx_ || cy_)) continue;
       const int64_t i0 = cx.rbase[0] + r0 + rr, i1 = cx.rbase[1] + r0 + rr;
+      // (false for NaN: excluded diagonals, windows that cannot match)
+      bool cx_, cy_;
+      if constexpr (kMat) {
+        cx_ = live && rv.x + mk.x > cx.thr;
+        cy_ = live && rv.y + mk.y > cx.thr;
+        if (cx_) cx_ = rv.x + mk.x > mat_cell_floor(cx, i0, i0 + jd);
+        if (cy_) cy_ = rv.y + mk.y > mat_cell_floor(cx, i1, i1 + jd);
+      } else {
+        const float2 rb = sm.r_best[r0 + rr];
+        const float2 cbv = sm.c_best[padc(rcs)];
+        cx_ = live && rv.x + mk.x > fminf(rb.x, cbv.x);
+        cy_ = live && rv.y + mk.y > fminf(rb.y, cbv.y);
+      }
+      if (!__any_sync(0xffffffffu, cx_ || cy_)) continue;
       nreq += push_requests(sm, cx, warp, lane, cx_, cy_, rv, mk, i0, i1, jd);
+      // (one cell's bound says nothing of a window's k-th best)
+      if (kMat || cx.knn_k) continue;
       if (cx_) publish_bound(sm, cx, rv.x - mk.x, i0, i0 + jd, r0 + rr, rcs, 0);
       if (cy_) publish_bound(sm, cx, rv.y - mk.y, i1, i1 + jd, r0 + rr, rcs, 1);
     }
@@ -891,11 +914,19 @@ __device__ __forceinline__ void raise_shared(float2& slot, unsigned x, unsigned 
 // the series).  The key carries no partner: its index field 0 loses every
 // tie, and the cell the bound came from has a larger r (its own FP32 value
 // in the mixed form), so a real cell replaces it.
+// k-best lists (k > 0): every call's bound comes from cells of its own (a
+// row's in one band, a column's in one unit), so a list of the largest k
+// bounds holds a lower bound of the k-th best.
 __device__ __forceinline__ void raise_bound(uint64_t* keys, int64_t w, float lb,
-                                            const KeyLayout& kl) {
+                                            const KeyLayout& kl, int k) {
   if (!keys || !(lb > 0.f)) return;
   const uint64_t key = q_from_float_bits(__float_as_uint(lb), kl.frac_bits) << kl.idx_bits;
-  if (key > __ldcg(keys + w)) atomicMax(reinterpret_cast<u64*>(keys + w), key);
+  if (k > 0) {
+    u64* list = reinterpret_cast<u64*>(keys + w * k);
+    if (key > __ldcg(list + k - 1)) topk_insert(list, k, key);
+  } else if (key > __ldcg(keys + w)) {
+    atomicMax(reinterpret_cast<u64*>(keys + w), key);
+  }
 }
 
 // MATRIX_SUMMARY: a thread's running maxima (per segment and target).
@@ -903,18 +934,6 @@ struct MatRun {
   int cell[2][2];
   float mx[2][2];
 };
-
-// Order-preserving uint32 image of a float (not NaN).
-__device__ __forceinline__ unsigned ord_float(float x) {
-  const unsigned b = __float_as_uint(x);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-// n / d for n < 2^32 and d >= 2 from M = ceil(2^64 / d): exact while
-// n d < 2^64 (floor(n M / 2^64) = n / d + n e / (d 2^64), e = M d - 2^64 < d).
-__device__ __forceinline__ int64_t div_magic(int64_t n, uint64_t M) {
-  return static_cast<int64_t>(__umul64hi(static_cast<uint64_t>(n), M));
-}
 
 // MATRIX_SUMMARY: a thread-step whose block crosses a grid boundary (flags
 // fx, fy per segment) is walked again from the step's start (rewound from
@@ -984,17 +1003,19 @@ __device__ __noinline__ void mat_cells_block(Smem& sm, const float2 (&cov_end)[k
 // kExact selects the FP64 1NN form: the FP32 arithmetic only rules cells out,
 // by the deterministic bound E (kStepCov ...), and every other cell's r is
 // computed in FP64 (verify_exact_kernel).
-// kBound selects the bounds pass of a 1NN form: every cell raises its row's
-// and its column's best to its FP32 r less the step's margin, a bound with no
-// partner (no candidate is looked at, nothing is verified).
+// kBound selects the bounds pass: every cell raises its row's and its
+// column's best (kMat: its grid entry) to its FP32 r less the step's margin,
+// a bound with no partner (no candidate is looked at, nothing is verified).
 template <bool kSum, bool kCoarse, bool kMat = false, bool kKnn = false, bool kExact = false,
           bool kBound = false>
 __device__ __forceinline__ void band_body(const JoinParams& P) {
   static_assert(!(kMat && (kSum || kCoarse)), "the matrix form takes per-cell maxima");
   static_assert(!(kKnn && (kSum || kCoarse || kMat)), "the k-best form is a 1NN variant");
-  static_assert(!(kExact && (kSum || kMat || kKnn)), "the exact form is a 1NN variant");
-  static_assert(!(kBound && (kSum || kCoarse || kMat || kKnn)), "bounds are for the 1NN forms");
-  constexpr bool kWindow = !kBound && !(kSum && !kCoarse);  // steps carry the column window
+  static_assert(!(kExact && (kSum || kKnn || kCoarse)), "no exact form of these");
+  static_assert(!(kBound && (kSum || kCoarse || kKnn || (kMat && !kExact))), "no bounds of these");
+  constexpr bool kRaise = kBound && !kMat;   // bounds of every window
+  constexpr bool kRuns = kMat && (!kExact || kBound);  // running maxima of grid entries
+  constexpr bool kWindow = !kRaise && !(kSum && !kCoarse);  // steps carry the column window
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int t = threadIdx.x;
@@ -1017,7 +1038,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
   static_assert(sizeof(MatRun) * kThreads <= sizeof(SlowItem) * kWarps * kQueue,
                 "matrix state exceeds the queue space");
   MatRun& mrun = reinterpret_cast<MatRun*>(&sm.queue[0][0])[t];
-  if constexpr (kMat) {
+  if constexpr (kRuns) {
 #pragma unroll
     for (int g = 0; g < 2; ++g)
 #pragma unroll
@@ -1048,7 +1069,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         sm.cx.budget = P.req_budget;
         sm.cx.wide_budget = P.wide_budget;
         if (!kBound && out_of_range && uu < P.total_units)
-          P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = uu;
+          P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = uu;  // (no request made)
       }
       if (uu < P.total_units) {
         int pi;
@@ -1070,11 +1091,24 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
     }
     if constexpr (kBound) {
-      // about 2^14 cells per window (uniform: sm.prob and sm.band are the
-      // unit's)
-      const int64_t longest = sm.prob.R.ns > sm.prob.C.ns ? sm.prob.R.ns : sm.prob.C.ns;
-      const int64_t stride = longest >> 14 > 1 ? longest >> 14 : 1;
-      if (sm.band % stride != stride - 1) {
+      // (uniform: sm.prob, sm.band and sm.unit_in_band are the unit's)
+      bool skip;
+      if constexpr (kMat) {
+        // rows of every grid entry: every second to eighth unit of a band
+        const int64_t span = P.rows_per_cell < P.cols_per_cell ? P.rows_per_cell : P.cols_per_cell;
+        int64_t stride = span / (2 * sm.prob.seg_len);
+        stride = stride < 1 ? 1 : (stride > 8 ? 8 : stride);
+        skip = sm.unit_in_band % stride != 0;
+      } else {
+        // about 2^14 cells per window; k-best lists: 4 k bands
+        const int64_t longest = sm.prob.R.ns > sm.prob.C.ns ? sm.prob.R.ns : sm.prob.C.ns;
+        int64_t stride = longest >> 14;
+        if (P.knn_k && stride > longest / (int64_t{4} * kBand * P.knn_k))
+          stride = longest / (int64_t{4} * kBand * P.knn_k);
+        if (stride < 1) stride = 1;
+        skip = sm.band % stride != stride - 1;
+      }
+      if (skip) {
         __syncthreads();
         continue;
       }
@@ -1323,10 +1357,11 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       cx.overflow = P.counters + 6;
       cx.sum_mode = kSum;
       cx.thr = static_cast<float>(P.threshold);
-      cx.knn_k = kKnn ? P.knn_k : 0;
+      cx.knn_k = kKnn || kExact ? P.knn_k : 0;
       if constexpr (kMat) {
         cx.mat = P.mat;
         cx.mat_w = P.mat_w;
+        cx.mat_h = P.mat_h;
         cx.rpc = P.rows_per_cell;
         cx.cpc = P.cols_per_cell;
         cx.rpc_magic = P.rpc_magic;
@@ -1344,7 +1379,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       // column, which flushes the previous one in its place)
       const int64_t left = seg_len[0] - q * kSlab;
       const int nsteps = left >= kSlab ? kSteps : static_cast<int>((left + 15) / 16) * 2;
-      const int ncols = (kSum || kBound) && q > 0 ? kCols : (kBand + nsteps * kRows + 31) / 32 * 32;
+      const int ncols = (kSum || kRaise) && q > 0 ? kCols : (kBand + nsteps * kRows + 31) / 32 * 32;
       int64_t rbase[2], rend[2], cbase_g[2];
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
@@ -1361,7 +1396,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       // consecutive columns or rows) at a time: per 8-column block and per
       // 8-row step the smallest best, the largest inverse norm and the
       // largest |df|, |dg|.
-      if (!sum_mode && !kBound && q > 0 && P.refresh_cols && pr.key_col) {
+      if (!sum_mode && !kRaise && q > 0 && P.refresh_cols && pr.key_col) {
         // Joins that start cold (no seeds): the columns kept from the last
         // slab take their bests from the profile keys, which other CTAs
         // raise quickly at the start; ring columns otherwise keep the bests
@@ -1401,12 +1436,12 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         // A window that cannot match (padding, NaN or flat) must not lower
         // the filter threshold: its best is "unreachable".
         float2 cbv;
-        if constexpr (kBound) {
+        if constexpr (kRaise) {
           // the previous occupant's bounds go to its keys
           if (q > 0) {
             const float2 old = sm.c_best[padc(rc)];
-            raise_bound(pr.key_col, j0 - kCols, old.x, P.kl);
-            raise_bound(pr.key_col, j1 - kCols, old.y, P.kl);
+            raise_bound(pr.key_col, j0 - kCols, old.x, P.kl, P.knn_k);
+            raise_bound(pr.key_col, j1 - kCols, old.y, P.kl, P.knn_k);
           }
           cbv = make_float2(0.f, 0.f);
         } else if (sum_mode) {
@@ -1458,7 +1493,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         f.w = ok1 ? pr.R.dg32[i1] : 0.f;
         const float2 iv = make_float2(ok0 ? pr.R.inv32[i0] : qnan(), ok1 ? pr.R.inv32[i1] : qnan());
         float2 rbv;
-        if (sum_mode || kBound) {
+        if (sum_mode || kRaise) {
           rbv = make_float2(0.f, 0.f);
         } else {
           rbv.x = (pr.key_row && ok0 && !isnan(iv.x)) ? best_floor(pr.key_row, i0) : kNoTarget;
@@ -1489,7 +1524,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       float2 ciw[16];
       // bounds pass: the last 7 columns' bounds of a step, its next step's first
       [[maybe_unused]] float2 cnext[kDiags - 1];
-      if constexpr (kBound) {
+      if constexpr (kRaise) {
 #pragma unroll
         for (int x = 0; x < kDiags - 1; ++x) cnext[x] = make_float2(0.f, 0.f);
       }
@@ -1550,7 +1585,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
 
         // fast path: recurrence + block maximum
         float bx = -3.f, by = -3.f;
-        if constexpr (kBound) {
+        if constexpr (kRaise) {
           // largest r of each row (over the thread's diagonals) and column
           float2 cmax[kRows + kDiags - 1];
           float4 cf[kRows + kDiags - 1];
@@ -1793,17 +1828,35 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             }
           }
         }
-        bool trig = bx > tx || by > ty;
-        if constexpr (kMat) {
+        [[maybe_unused]] bool trig = bx > tx || by > ty;
+        if constexpr (kMat && kExact && !kBound) {
+          // exact matrix: a block that may hold a grid entry's largest r, by
+          // the bounds of the entries it touches (two each way at most)
+          trig = false;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const float ub = (g ? by : bx) + fmaf(kBoundSlack, g ? mg.y : mg.x, kAbsSlack);
+            if (!(ub > thr)) continue;
+            const int64_t i0 = rbase[g] + r0, j0 = i0 + d_my;
+            float lo = kNoTarget;
+            if (sm.cx.mcol) lo = mat_block_floor(sm.cx, i0, kRows - 1, j0, kRows + kDiags - 2);
+            if (sm.cx.mrow)
+              lo = fminf(lo, mat_block_floor(sm.cx, j0, kRows + kDiags - 2, i0, kRows - 1));
+            trig = trig || ub > lo;
+          }
+        } else if constexpr (kMat) {
           // a block inside one grid entry (per target) raises the thread's
           // running maximum of that entry, published when the thread's
           // blocks move on; a block across a grid boundary routes each cell
           trig = false;
-          const float2 smg = mul2(make_float2(kStepMarginC, kStepMarginC), mg);
+          const float2 smg = mul2(make_float2(kMg, kMg), mg);
+          // the exact form's bounds lie E below the values
+          const float2 sub = kExact ? make_float2(smg.x + kAbsSlack, smg.y + kAbsSlack)
+                                    : make_float2(0.f, 0.f);
           bool nonuni[2] = {false, false};
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
-            const float bm = g ? by : bx;
+            const float bm = (g ? by : bx) - (g ? sub.y : sub.x);
             if (!(bm > thr)) continue;
             tfast = fmaxf(tfast, g ? smg.y : smg.x);
             const int64_t i0 = rbase[g] + r0, j0 = i0 + d_my;
@@ -1839,7 +1892,10 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
               }
             }
           }
-          if (nonuni[0] || nonuni[1]) mat_cells_block(sm, cov, s, t, nonuni[0], nonuni[1]);
+          // (the bounds pass does without the blocks across a boundary: their
+          // cells one by one took two thirds of its time)
+          if (!kBound && (nonuni[0] || nonuni[1]))
+            mat_cells_block(sm, cov, s, t, nonuni[0], nonuni[1]);
         }
         // segments the exact path walks (bit 0: first, bit 1: second)
         [[maybe_unused]] int smask = 3;
@@ -1930,7 +1986,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         const unsigned pmask = __ballot_sync(0xffffffffu, pend >= 0);
         if (pmask || qn >= kQueue / 2 || (qn && s + 2 == nsteps)) {
           if (qn) {
-            n_verify += kExact ? drain_exact(sm, warp, qn, lane)
+            n_verify += kExact ? drain_exact<kMat>(sm, warp, qn, lane)
                                : drain_queue<!kCoarse>(sm, warp, qn, lane);
             qn = 0;
           }
@@ -1946,13 +2002,13 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
               it.owner = t;
             }
             const int take = (np - done) < kQueue ? (np - done) : kQueue;
-            n_verify += kExact ? drain_exact(sm, warp, take, lane)
+            n_verify += kExact ? drain_exact<kMat>(sm, warp, take, lane)
                                : drain_queue<!kCoarse>(sm, warp, take, lane);
           }
           pend = -1;
         }
       }
-      if constexpr (kBound) {
+      if constexpr (kRaise) {
         // the columns after the last step's first 8
         const int rb = (rq + nsteps + t) < kBlocks ? (rq + nsteps + t) : (rq + nsteps + t - kBlocks);
 #pragma unroll
@@ -1960,13 +2016,13 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
           raise_shared(sm.c_best[9 * rb + x], __float_as_uint(cnext[x].x), __float_as_uint(cnext[x].y));
         __syncthreads();
         const float2 v = sm.r_best[t];
-        raise_bound(pr.key_row, rbase[0] + t, v.x, P.kl);
-        raise_bound(pr.key_row, rbase[1] + t, v.y, P.kl);
+        raise_bound(pr.key_row, rbase[0] + t, v.x, P.kl, P.knn_k);
+        raise_bound(pr.key_row, rbase[1] + t, v.y, P.kl, P.knn_k);
         if (q + 1 == nslabs) {
           for (int c = t; c < ncols; c += kThreads) {
             const float2 u = sm.c_best[padc(ringc(ring0, c))];
-            raise_bound(pr.key_col, cbase_g[0] + c, u.x, P.kl);
-            raise_bound(pr.key_col, cbase_g[1] + c, u.y, P.kl);
+            raise_bound(pr.key_col, cbase_g[0] + c, u.x, P.kl, P.knn_k);
+            raise_bound(pr.key_col, cbase_g[1] + c, u.y, P.kl, P.knn_k);
           }
           __syncthreads();  // sm.prob is read above
         }
@@ -1974,7 +2030,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
       n_steps += nsteps;
       __syncthreads();
-      if constexpr (kExact) {
+      if constexpr (kExact && !kBound) {
         // A unit whose cells its FP32 values cannot rule out (error bounds
         // above the spread of the correlations: near-flat windows beside
         // large steps, exact repeats everywhere) is left to the FP64 band
@@ -1982,7 +2038,10 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
         const bool leave = sm.cx.unit_lost;
         __syncthreads();
         if (leave) {
-          if (t == 0) P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = u;
+          if (t == 0) {
+            P.fp64_list[atomicAdd(P.fp64_count, 1ull)] = u;
+            P.fp64_unit[u] = 1;
+          }
           break;
         }
       }
@@ -2025,14 +2084,14 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
     atomicAdd(P.counters + 1, n_slow);
     atomicAdd(P.counters + 2, n_verify);
   }
-  if constexpr (kMat) {
+  if constexpr (kRuns) {
 #pragma unroll
     for (int g = 0; g < 2; ++g)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         if (mrun.cell[g][h] >= 0) atomicMax(P.mat + mrun.cell[g][h], ord_float(mrun.mx[g][h]));
   }
-  if constexpr (kSum || kMat) {
+  if constexpr (kSum || (kMat && !kExact)) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tfast = fmaxf(tfast, __shfl_xor_sync(0xffffffffu, tfast, o));
     if (lane == 0 && P.counters && tfast > 0.f)
@@ -2074,6 +2133,25 @@ __global__ void __launch_bounds__(kThreads, 4) join_exact_1nn_kernel(JoinParams 
 
 __global__ void __launch_bounds__(kThreads, 4) bound_exact_1nn_kernel(JoinParams P) {
   band_body<false, false, false, false, true, true>(P);
+}
+
+__global__ void __launch_bounds__(kThreads, 4) join_exact_mat_kernel(JoinParams P) {
+  band_body<false, false, true, false, true>(P);
+}
+
+__global__ void __launch_bounds__(kThreads, 4) bound_exact_mat_kernel(JoinParams P) {
+  band_body<false, false, true, false, true, true>(P);
+}
+
+__global__ void knn_floor_kernel(const unsigned long long* __restrict__ bounds,
+                                 const unsigned long long* __restrict__ lists, int64_t n, int k,
+                                 double thr, KeyLayout kl, uint64_t* __restrict__ out) {
+  const int64_t w = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (w >= n) return;
+  const uint64_t a = bounds[w * k + k - 1] >> kl.idx_bits, b = lists[w * k + k - 1] >> kl.idx_bits;
+  const uint64_t c = q_from_float_bits(__float_as_uint(__double2float_rd(thr)), kl.frac_bits);
+  const uint64_t q = a > b ? (a > c ? a : c) : (b > c ? b : c);
+  out[w] = q << kl.idx_bits;
 }
 
 __global__ void __launch_bounds__(kThreads, 4) bound_mixed_1nn_kernel(JoinParams P) {

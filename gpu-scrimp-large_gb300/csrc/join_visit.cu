@@ -34,12 +34,6 @@ namespace {
 
 constexpr int kVisitThreads = 256;  // one diagonal per thread
 
-// Order-preserving uint32 image of a float (NaN excluded by the callers).
-__device__ __forceinline__ unsigned ord_float(float x) {
-  const unsigned b = __float_as_uint(x);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
 __device__ __forceinline__ double seed_dot(const SeriesDev& R, const SeriesDev& C,
                                            int64_t i, int64_t j, int64_t m) {
   const double mr = R.mean[i], mc = C.mean[j];
@@ -53,14 +47,6 @@ __device__ __forceinline__ double seed_dot(const SeriesDev& R, const SeriesDev& 
   }
   for (; t < m; ++t) s0 = fma(R.T[i + t] - mr, C.T[j + t] - mc, s0);
   return (s0 + s1) + (s2 + s3);
-}
-
-__device__ __forceinline__ void topk_insert(unsigned long long* slots, int k,
-                                            unsigned long long key) {
-  for (int s = 0; s < k && key != 0; ++s) {
-    const unsigned long long old = atomicMax(slots + s, key);
-    if (old < key) key = old;  // the displaced key moves on
-  }
 }
 
 // x / div and x % div of a position that advances by one.
@@ -103,18 +89,23 @@ join_visit_kernel(JoinParams P, VisitArgs V) {
   __shared__ long long s_unit;
   const int t = threadIdx.x;
   const double thr = P.threshold;
+  // the whole queue, or quarter bands of the units the exact form left
+  constexpr int kQuarters = 4;
+  const bool listed = P.fp64_list != nullptr;
+  const int64_t total_units =
+      listed ? kQuarters * static_cast<int64_t>(*P.fp64_count) : P.total_units;
   for (;;) {
     if (t == 0) s_unit = static_cast<long long>(atomicAdd(P.unit_counter, 1ull));
     __syncthreads();
     const int64_t u = s_unit;
     __syncthreads();
-    if (u >= P.total_units) break;
+    if (u >= total_units) break;
     int pi;
     int64_t band, ub;
-    decode_unit(P, u, &pi, &band, &ub);
+    decode_unit(P, listed ? P.fp64_list[u / kQuarters] : u, &pi, &band, &ub);
     const Problem& pr = P.prob[pi];
     const int64_t K = P.seg_len;
-    const int64_t D0 = pr.d_lo + band * kVisitThreads;
+    const int64_t D0 = pr.d_lo + band * P.band_width + (listed ? u % kQuarters * kVisitThreads : 0);
     const int64_t d = D0 + t;
     if (d >= pr.d_hi || (d >= pr.x_lo && d < pr.x_hi)) continue;
     const int64_t rows_b = band_rows(pr.R.ns, pr.C.ns, D0);
@@ -183,8 +174,7 @@ __global__ void ord_to_floats_kernel(const unsigned* __restrict__ in, float* __r
                                      int64_t n) {
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
-  const unsigned b = in[i];
-  out[i] = __uint_as_float((b & 0x80000000u) ? (b & 0x7FFFFFFFu) : ~b);
+  out[i] = float_of_ord(in[i]);
 }
 
 }  // namespace scamp_gb300
