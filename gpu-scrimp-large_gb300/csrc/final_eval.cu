@@ -216,14 +216,17 @@ __global__ void __launch_bounds__(256) verify_exact_kernel(JoinParams P) {
   const unsigned long long total = P.counters[3];
   const int64_t n = total < static_cast<unsigned long long>(P.vreq_cap)
                         ? static_cast<int64_t>(total) : P.vreq_cap;
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
   constexpr int kGroups = 32 / kLanes;
   const int k = P.knn_k;
   const bool plain = k == 0 && !P.mat;
   const bool some_left = *P.fp64_count > 0;
   const float thr = plain ? -3.f : __double2float_rd(P.threshold);
-  for (int64_t g0 = ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups;
-       g0 < n; g0 += nwarps * kGroups) {
+  // a block takes 64 requests in a row (verify_requests_kernel)
+  constexpr int kRun = 64;
+  const int step = (blockDim.x >> 5) * kGroups;
+  for (int64_t run = static_cast<int64_t>(blockIdx.x) * kRun; run < n;
+       run += static_cast<int64_t>(gridDim.x) * kRun)
+  for (int64_t g0 = run + (threadIdx.x >> 5) * kGroups; g0 < run + kRun && g0 < n; g0 += step) {
     const int64_t g = g0 + lane / kLanes;
     const VerifyReq rq = P.vreq[g < n ? g : g0];
     const int p = static_cast<int>(rq.i >> 40);

@@ -162,6 +162,11 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // PTX sqrt.approx.f32: an approximate square root (a few ulp); sqrt(0) = 0.
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
@@ -263,7 +268,7 @@ struct Smem {
   long long unit, band, unit_in_band;
   int prob_index;
   SlowCtx cx;
-  // exact form: each warp's block of the request buffer and its used slots
+  // each warp's block of the request buffer and its used slots
   unsigned long long rq_base[kWarps];
   int rq_used[kWarps];
 };
@@ -383,24 +388,39 @@ __device__ __forceinline__ float cov_part(const SeriesDev& R, const SeriesDev& C
 }
 
 // The same covariance computed by a whole warp: lane l sums the terms
-// t = l, l + 32, ...; the partial sums meet in a shuffle reduction.
+// t = l, l + 32, ...; the partial sums meet in a shuffle reduction.  The
+// samples' centring terms belong to their blocks, of which a window touches
+// 18 at most (block_shift()): each lane forms one block's, and a sample's
+// comes by a shuffle (loaded and formed again for every sample, the seeds of
+// 2^20 windows of m = 1024 took 2.19 ms, now 0.89: 9.3 TB/s from L2).
 __device__ __forceinline__ float verify_cov_warp(const SeriesDev& R, const SeriesDev& C,
                                                  int64_t i, int64_t j, int64_t m, int lane) {
-  const int sh = R.bshift;
+  const int sh = R.bshift, mi = static_cast<int>(m);
   const int64_t bi = i >> sh, bj = j >> sh;
   const float mri = R.mu_rel[i], mcj = C.mu_rel[j];
-  const float hr0 = R.bhi[bi], lr0 = R.blo[bi], hc0 = C.bhi[bj], lc0 = C.blo[bj];
+  // windows start oi, oj samples into their blocks
+  const int oi = static_cast<int>(i - (bi << sh)), oj = static_cast<int>(j - (bj << sh));
+  const int br = lane < ((oi + mi - 1) >> sh) + 1 ? lane : 0;
+  const int bc = lane < ((oj + mi - 1) >> sh) + 1 ? lane : 0;
+  const float xb = ((R.bhi[bi + br] - R.bhi[bi]) + (R.blo[bi + br] - R.blo[bi])) - mri;
+  const float yb = ((C.bhi[bj + bc] - C.bhi[bj]) + (C.blo[bj + bc] - C.blo[bj])) - mcj;
+  const float* __restrict__ tr = R.T32 + i;
+  const float* __restrict__ tc = C.T32 + j;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int64_t t0 = lane; t0 < m; t0 += 128) {
+  for (int t0 = lane; t0 - lane < mi; t0 += 128) {
+    float x[4], y[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int64_t t = t0 + 32 * u;
-      if (t < m) {
-        const int64_t br = (i + t) >> sh, bc = (j + t) >> sh;
-        const float x = R.T32[i + t] + (((R.bhi[br] - hr0) + (R.blo[br] - lr0)) - mri);
-        const float y = C.T32[j + t] + (((C.bhi[bc] - hc0) + (C.blo[bc] - lc0)) - mcj);
-        acc[u] = fmaf(x, y, acc[u]);
-      }
+      const int t = t0 + 32 * u;
+      x[u] = t < mi ? tr[t] : 0.f;
+      y[u] = t < mi ? tc[t] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = t0 + 32 * u;
+      const float dx = __shfl_sync(0xffffffffu, xb, (oi + t) >> sh);
+      const float dy = __shfl_sync(0xffffffffu, yb, (oj + t) >> sh);
+      if (t < mi) acc[u] = fmaf(x[u] + dx, y[u] + dy, acc[u]);
     }
   }
   float a = (acc[0] + acc[1]) + (acc[2] + acc[3]);
@@ -506,6 +526,37 @@ __device__ __forceinline__ void exact_cell(Smem& sm, const SlowCtx& cx, float rv
   }
 }
 
+// The unused slots of the warp's block of the request buffer
+// become requests that rule themselves out.
+__device__ __forceinline__ void close_requests(Smem& sm, const SlowCtx& cx, int warp, int lane) {
+  const unsigned long long base = sm.rq_base[warp];
+  for (int s = sm.rq_used[warp] + lane; s < kReqChunk; s += 32)
+    if (base + s < static_cast<unsigned long long>(cx.vcap)) cx.vreq[base + s] = VerifyReq{0, 0, -4.f};
+}
+
+// n consecutive slots of the request buffer for the warp, from a block of
+// kReqChunk that it takes at a time, so that the global counter's round trip
+// is paid once per block and not once per row of candidates.  Called by the
+// whole warp, n <= kReqChunk.
+__device__ __forceinline__ unsigned long long take_requests(Smem& sm, const SlowCtx& cx, int warp,
+                                                            int lane, int n) {
+  int used = sm.rq_used[warp];
+  unsigned long long base = sm.rq_base[warp];
+  if (used + n > kReqChunk) {
+    close_requests(sm, cx, warp, lane);
+    if (lane == 0) base = atomicAdd(cx.vcount, static_cast<unsigned long long>(kReqChunk));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    used = 0;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    sm.rq_base[warp] = base;
+    sm.rq_used[warp] = used + n;
+  }
+  __syncwarp();
+  return base + used;
+}
+
 // Exact path of queued blocks, 8 lanes per block (four blocks per pass):
 // lane k holds the covariances of diagonal k in both segments (an f32x2
 // pair, as the fast path holds them) at the block's end and visits the
@@ -593,11 +644,7 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
       const unsigned mx = __ballot_sync(0xffffffffu, qx), my = __ballot_sync(0xffffffffu, qy);
       unsigned long long sx = 0, sy = 0;
       if (mx | my) {
-        const int leader = __ffs(mx | my) - 1;
-        unsigned long long base = 0;
-        if (lane == leader)
-          base = atomicAdd(cx.vcount, static_cast<unsigned long long>(__popc(mx) + __popc(my)));
-        base = __shfl_sync(0xffffffffu, base, leader);
+        const unsigned long long base = take_requests(sm, cx, warp, lane, __popc(mx) + __popc(my));
         const unsigned lt = (1u << lane) - 1u;
         sx = base + __popc(mx & lt) + __popc(my & lt);
         sy = sx + (qx ? 1u : 0u);
@@ -639,38 +686,21 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
   return nreq;
 }
 
-// Exact form: the unused slots of the warp's block of the request buffer
-// become requests that rule themselves out.
-__device__ __forceinline__ void close_requests(Smem& sm, const SlowCtx& cx, int warp, int lane) {
-  const unsigned long long base = sm.rq_base[warp];
-  for (int s = sm.rq_used[warp] + lane; s < kReqChunk; s += 32)
-    if (base + s < static_cast<unsigned long long>(cx.vcap)) cx.vreq[base + s] = VerifyReq{0, 0, -4.f};
-}
-
 // Exact form: writes the requests of the lanes that qx, qy mark (segments x
-// and y of cells (i, i + d)) into the warp's block of the request buffer,
-// kReqChunk slots taken at a time, so that the global counter's round trip is
-// paid once per block and not once per row of candidates.  Called by the
-// whole warp; returns the number written.
+// and y of cells (i, i + d)).  Called by the whole warp; returns the number
+// written.
 __device__ __forceinline__ int push_requests(Smem& sm, const SlowCtx& cx, int warp, int lane,
                                              bool qx, bool qy, float2 rv, float2 mk, int64_t ix,
                                              int64_t iy, int64_t d) {
   const unsigned mx = __ballot_sync(0xffffffffu, qx), my = __ballot_sync(0xffffffffu, qy);
   const int n = __popc(mx) + __popc(my);
   if (n == 0) return 0;
-  int used = sm.rq_used[warp];
-  unsigned long long base = sm.rq_base[warp];
-  if (used + n > kReqChunk) {
-    close_requests(sm, cx, warp, lane);
-    if (lane == 0) base = atomicAdd(cx.vcount, static_cast<unsigned long long>(kReqChunk));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    used = 0;
-  }
+  const unsigned long long base = take_requests(sm, cx, warp, lane, n);
   const unsigned lt = (1u << lane) - 1u;
   VerifyReq rq;
   rq.d = static_cast<uint32_t>(d);
-  const unsigned long long sx = base + used + __popc(mx & lt);
-  const unsigned long long sy = base + used + __popc(mx) + __popc(my & lt);
+  const unsigned long long sx = base + __popc(mx & lt);
+  const unsigned long long sy = base + __popc(mx) + __popc(my & lt);
   if (qx && sx < static_cast<unsigned long long>(cx.vcap)) {
     rq.i = static_cast<uint64_t>(ix) | (static_cast<uint64_t>(cx.prob) << 40);
     rq.ub = rv.x + mk.x;
@@ -683,14 +713,11 @@ __device__ __forceinline__ int push_requests(Smem& sm, const SlowCtx& cx, int wa
   }
   const unsigned wide = __popc(__ballot_sync(0xffffffffu, qx && mk.x > kWideBound)) +
                         __popc(__ballot_sync(0xffffffffu, qy && mk.y > kWideBound));
-  if (lane == 0) {
-    sm.rq_base[warp] = base;
-    sm.rq_used[warp] = used + n;
-    if (atomicAdd(&sm.cx.unit_reqs, static_cast<unsigned>(n)) + n > cx.budget ||
-        (wide && atomicAdd(&sm.cx.unit_wide, wide) + wide > cx.wide_budget) ||
-        base + used + n > static_cast<unsigned long long>(cx.vcap))
-      sm.cx.unit_lost = 1;
-  }
+  if (lane == 0 &&
+      (atomicAdd(&sm.cx.unit_reqs, static_cast<unsigned>(n)) + n > cx.budget ||
+       (wide && atomicAdd(&sm.cx.unit_wide, wide) + wide > cx.wide_budget) ||
+       base + n > static_cast<unsigned long long>(cx.vcap)))
+    sm.cx.unit_lost = 1;
   __syncwarp();
   return n;
 }
@@ -1048,14 +1075,14 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       }
   }
 
+  if (lane == 0) sm.rq_used[warp] = kReqChunk;  // no block of requests yet
+  __syncwarp();
   // exact form: series out of FP32's safe range leave every unit to the FP64
   // band kernel
   bool out_of_range = false;
   if constexpr (kExact) {
     const float vmax = __uint_as_float(P.range[0]), imax = __uint_as_float(P.range[1]);
     out_of_range = !(vmax <= kExactMaxValue && imax <= kExactMaxInv && vmax * imax <= kExactMaxRatio);
-    if (lane == 0) sm.rq_used[warp] = kReqChunk;  // no block yet
-    __syncwarp();
   }
 
   for (;;) {
@@ -1709,15 +1736,22 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             const float2 dfr = make_float2(rf.x, rf.y), dgr = make_float2(rf.z, rf.w);
             const float2 ivr = sm.r_iv[r0 + rr];
             rsum[rr] = make_float2(0.f, 0.f);
+            float2 rodd;  // the previous diagonal's r (k odd)
 #pragma unroll
             for (int k = 0; k < kDiags; ++k) {
               const int x = rr + k;
               const int slot = base + x + (x >> 3);
               const float4 c4 = col_fg(sm, slot);
               const float2 r2 = mul2(mul2(cov[k], sm.u.s.c_iv[slot]), ivr);
-              bx = fmaxf(bx, r2.x);  // NaN cells are ignored
-              by = fmaxf(by, r2.y);
-              dmin = make_float2(fminf(dmin.x, fabsf(r2.x - thr)), fminf(dmin.y, fabsf(r2.y - thr)));
+              // (two cells per three-input instruction; NaN cells are ignored)
+              if (k & 1) {
+                bx = max3(bx, rodd.x, r2.x);
+                by = max3(by, rodd.y, r2.y);
+                dmin = make_float2(min3(dmin.x, fabsf(rodd.x - thr), fabsf(r2.x - thr)),
+                                   min3(dmin.y, fabsf(rodd.y - thr), fabsf(r2.y - thr)));
+              } else {
+                rodd = r2;
+              }
               const float ax = r2.x > thx ? r2.x : 0.f;
               const float ay = r2.y > thy ? r2.y : 0.f;
               rsum[rr] = make_float2(rsum[rr].x + ax, rsum[rr].y + ay);
@@ -2066,7 +2100,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       if (sum_mode && q + 1 == nslabs) __syncthreads();
     }
   }
-  if constexpr (kExact && !kBound) {
+  if constexpr (!kBound && !kRuns) {
     __syncwarp();
     sm.cx.vcap = P.vreq_cap;  // (a CTA without a unit has no context; every writer the same)
     sm.cx.vreq = P.vreq;
@@ -2107,7 +2141,10 @@ __global__ void __launch_bounds__(kThreads, 4) join_mixed_1nn_kernel(JoinParams 
   band_body<false, false>(P);
 }
 
-__global__ void __launch_bounds__(kThreads, 4) join_mixed_sum_kernel(JoinParams P) {
+// (three CTAs per SM: with the registers of four, 220 bytes spilled per
+// thread; 200003 samples, m = 256, r > 0.5 18.8 -> 17.6 ms, m = 100, r > 0.9
+// 15.1 -> 13.3)
+__global__ void __launch_bounds__(kThreads, 3) join_mixed_sum_kernel(JoinParams P) {
   band_body<true, false>(P);
 }
 
@@ -2171,14 +2208,20 @@ verify_requests_kernel(JoinParams P) {
   const unsigned long long total = P.counters[3];
   const int64_t n = total < static_cast<unsigned long long>(P.vreq_cap)
                         ? static_cast<int64_t>(total) : P.vreq_cap;
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-       w < n; w += nwarps) {
+  // A block takes kReqChunk requests in a row, what one warp of the join
+  // wrote: cells of neighbouring windows, whose samples its warps share in L1
+  // (one dot of m = 1024 reads 8 KB, from L2 the kernel's bound: 9.3e6
+  // requests 10.9 -> 8.9 ms, 2^18 x 2^17 windows of m = 256 0.91 -> 0.79 ms)
+  const int nwarps = blockDim.x >> 5;
+  for (int64_t w0 = static_cast<int64_t>(blockIdx.x) * kReqChunk; w0 < n;
+       w0 += static_cast<int64_t>(gridDim.x) * kReqChunk)
+  for (int64_t w = w0 + (threadIdx.x >> 5); w < w0 + kReqChunk && w < n; w += nwarps) {
     const VerifyReq rq = P.vreq[w];
     const Problem& pr = problem_of(P, static_cast<int>(rq.i >> 40));
     const int64_t i = static_cast<int64_t>(rq.i & ((uint64_t{1} << 40) - 1));
     const int64_t j = i + rq.d;
     if (P.profile_type == 2) {  // SUM_THRESH: the cell counts if above it
+      if (rq.ub < -3.f) continue;  // an unused slot
       const float cv = verify_cov_warp(pr.R, pr.C, i, j, pr.m, lane);
       const float rv = (cv * pr.C.inv32[j]) * pr.R.inv32[i];
       if (lane == 0 && rv > static_cast<float>(P.threshold)) {
