@@ -3,25 +3,29 @@
 // run behind the FP32 filter.
 //
 // Both join forms choose each window's best partner from a recurrence (FP64
-// in the plain form, FP32 behind a filter in the mixed form).  Before the
+// in the plain form, FP32 behind a filter in the others).  Before the
 // profile is written back, this kernel recomputes the correlation of every
-// (window, reported partner) pair directly: centred FP64 dot product and
-// centred sums of squares of the two windows, r = dot / sqrt(sxx * syy), so
-// the value a join reports does not carry the recurrence's drift or the
-// statistics' rounding.  This is the reference's correlation formula
-// (src/cpu_kernels.cpp:166-171 with the norms of src/cpu_stats.cpp:85-97,
-// the brute-force ULTRA statistics) evaluated once per reported cell.
+// (window, reported partner) pair directly: the centred FP64 dot product
+// times the two windows' inverse norms (stats.cu: compensated sums of
+// squares), so the value a join reports does not carry the recurrence's
+// drift.  This is the reference's correlation formula
+// (src/cpu_kernels.cpp:166-171 with the norms of src/cpu_stats.cpp:85-97)
+// evaluated once per reported cell.  Bound by the FP64 pipe at 3 operations
+// per sample (with the sums of squares formed again for every pair, 5:
+// 2^20 windows of m = 1024 9.8 -> 6.0 ms).
 //
 // Error bound (per reported value, against the exact correlation of the two
-// FP64 windows): every centred term x_t = fl(T - mu) carries one rounding;
-// each of a group's 8 lanes sums its terms by FMA into two accumulators of
-// at most ceil(m / 16) terms, one add joins them, three shuffle levels add
-// the lanes' sums, and the quotient takes three more roundings, so with
-// gamma_k = k u / (1 - k u), u = 2^-53:
-//   |r_hat - r| <= 2 gamma_{ceil(m/16) + 10}
-// (the dot's error is gamma_k * sum |x y| <= gamma_k ||x|| ||y||; each sum of
-// squares is off by at most gamma_k of itself).  The 64-bit key then keeps r
-// to 2^-F.  The host adds the two (final_eval_bound).
+// FP64 windows), u = 2^-53, gamma_k = k u / (1 - k u): every centred term
+// x_t = fl(T - mu) carries one rounding; each of a group's 8 lanes sums its
+// terms by FMA into two accumulators of at most ceil(m / 16) terms, one add
+// joins them and three shuffle levels add the lanes' sums, so the dot is off
+// by gamma_{ceil(m/16) + 6} ||x|| ||y||; an inverse norm by 5 u at
+// most (its sum of squares is compensated throughout; then its rounding, a
+// square root and a quotient); two products follow.
+// Together at most gamma_{ceil(m/16) + 18}, within the stated
+//   |r_hat - r| <= 2 gamma_{ceil(m/16) + 10}.
+// The 64-bit key then keeps r to 2^-F.  The host adds the two
+// (final_eval_bound).
 //
 // Entries the join did not change (a best-so-far entry given on input, whose
 // index may refer to another join) are left as they are.
@@ -34,46 +38,6 @@ namespace scamp_gb300 {
 namespace {
 
 constexpr int kLanes = 8;  // lanes per window: four windows per warp
-
-// Direct FP64 correlation of window i of X with window j of Y by kLanes
-// lanes (a lane sums every kLanes-th term, the partial sums meet in a
-// shuffle tree); the value is valid in the group's first lane (NaN when a
-// window has no spread).
-__device__ __forceinline__ double corr_group_fp64(const SeriesDev& X, const SeriesDev& Y,
-                                                  int64_t i, int64_t j, int64_t m, int sub,
-                                                  bool first) {
-  const double mx = X.mean[i], my = Y.mean[j];
-  const double* __restrict__ tx = X.T + i;
-  const double* __restrict__ ty = Y.T + j;
-  double sxy = 0.0, sxx = 0.0, syy = 0.0, sxy2 = 0.0, sxx2 = 0.0, syy2 = 0.0;
-  int64_t t = sub;
-  for (; t + kLanes < m; t += 2 * kLanes) {
-    const double x0 = tx[t] - mx, y0 = ty[t] - my;
-    const double x1 = tx[t + kLanes] - mx, y1 = ty[t + kLanes] - my;
-    sxy = fma(x0, y0, sxy);
-    sxx = fma(x0, x0, sxx);
-    syy = fma(y0, y0, syy);
-    sxy2 = fma(x1, y1, sxy2);
-    sxx2 = fma(x1, x1, sxx2);
-    syy2 = fma(y1, y1, syy2);
-  }
-  if (t < m) {
-    const double x0 = tx[t] - mx, y0 = ty[t] - my;
-    sxy = fma(x0, y0, sxy);
-    sxx = fma(x0, x0, sxx);
-    syy = fma(y0, y0, syy);
-  }
-  sxy += sxy2;
-  sxx += sxx2;
-  syy += syy2;
-#pragma unroll
-  for (int o = kLanes / 2; o > 0; o >>= 1) {
-    sxy += __shfl_xor_sync(0xffffffffu, sxy, o);
-    sxx += __shfl_xor_sync(0xffffffffu, sxx, o);
-    syy += __shfl_xor_sync(0xffffffffu, syy, o);
-  }
-  return first ? sxy / sqrt(sxx * syy) : 0.0;
-}
 
 // Direct FP64 covariance of window i of X with window j of Y by kLanes lanes,
 // times the two windows' inverse norms; valid in every lane of the group.
@@ -128,8 +92,7 @@ __device__ __forceinline__ void eval_window(const EvalSide& s, int64_t w, int64_
   if (j < 0 || j >= s.Y.ns) k = 0;
   // groups with nothing to do still take part in the shuffles (no terms)
   const bool work = k != 0;
-  const double r = corr_group_fp64(s.X, s.Y, work ? w : 0, work ? j : 0, work ? m : 0, sub,
-                                   sub == 0);
+  const double r = corr_group_norms(s.X, s.Y, work ? w : 0, work ? j : 0, work ? m : 0, sub);
   if (sub == 0 && work && !isnan(r)) {
     // |r| <= 1 up to rounding; the key holds r in [-2, 2)
     const double rc = r > 1.0 ? 1.0 : (r < -1.0 ? -1.0 : r);
@@ -178,8 +141,7 @@ __global__ void __launch_bounds__(256) knn_final_eval_kernel(EvalSide S, int k, 
       }
       const int64_t j = key ? key_to_index(key, kl) : 0;
       const bool work = key != 0 && j >= 0 && j < S.Y.ns;
-      const double r = corr_group_fp64(S.X, S.Y, work ? w : 0, work ? j : 0, work ? S.m : 0, sub,
-                                       sub == 0);
+      const double r = corr_group_norms(S.X, S.Y, work ? w : 0, work ? j : 0, work ? S.m : 0, sub);
       if (sub == 0 && work) {
         const double rc = r > 1.0 ? 1.0 : (r < -1.0 ? -1.0 : r);
         list[s] = (!isnan(r) && r > thr)

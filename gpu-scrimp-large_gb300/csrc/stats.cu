@@ -182,8 +182,14 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
   mean_of(ps, pc, mu0, mu0_lo);
   double ss = 0, sc = 0;
   for (int64_t t = lane; t < m; t += 32) {
-    const double v = clean(T_raw[w0 + t]) - mu0;
-    acc2(ss, sc, v * v);
+    // (x - mu)^2 as a compensated product too: what a spike in window w0
+    // rounds stays in the sums after it has left
+    double vh = clean(T_raw[w0 + t]), vl = 0;
+    acc2(vh, vl, -mu0);
+    vl -= mu0_lo;
+    const double p = vh * vh;
+    sc += fma(vh, vh, -p) + 2.0 * vh * vl;
+    acc2(ss, sc, p);
   }
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1)
