@@ -1013,7 +1013,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   // the join is too small to give every resident CTA ~8 units.
   int64_t K;
   const double cells_d = static_cast<double>(plan.cells);
-  const int64_t k_lb = static_cast<int64_t>(cells_d / (8.0 * resident * 2.0 * W));
+  // (the mixed form's rounding depends on its segments, which are cut for four
+  // CTAs per SM whatever the kernel's occupancy)
+  const int64_t k_ctas = kind == K_MIXED ? int64_t{4} * ws.sms : resident;
+  const int64_t k_lb = static_cast<int64_t>(cells_d / (8.0 * k_ctas * 2.0 * W));
   if (kind == K_MIXED) {
     K = a->anchor_interval > 0 ? a->anchor_interval
                                : (is_1nn ? default_anchor_interval(m) : short_anchor_interval(m));
