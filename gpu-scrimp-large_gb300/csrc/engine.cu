@@ -153,6 +153,18 @@ int64_t exact_segment(double cells, int64_t resident, int W, int slab, int64_t m
 // a flat stretch leaves FP32 nothing, so a few say that the unit is lost.
 constexpr int64_t kReqPerCells = 4;
 constexpr int64_t kWidePerCells = 1024;
+// Requests of a k-best join in all, per cell over the window length; the units
+// beyond them are left to the visit kernel, whose time grows with k.  No
+// budget per unit: a unit of dense matches, one insertion after the other,
+// costs the visit kernel milliseconds, its requests microseconds.  20011-sample
+// walks, m = 128 (whole calls): five best, with 8 requests per 1000 cells of a
+// unit 30 walks of 100 lost a unit or two and took 4.1 ms, now all 1.15; ten
+// best 10.0 (visit kernel) -> 1.7, twenty 16 -> 4.3, 64 46 -> 20.  Where no
+// bound separates the best cells (60000 samples of a square wave, m = 1000,
+// five best) all requests would take 195 ms, the visit kernel takes 43, this
+// both in part: 46.
+double list_reqs(int64_t k) { return 3.0 + 0.75 * static_cast<double>(k); }
+constexpr int64_t kMaxListReqs = int64_t{1} << 27;  // 2 GiB of requests
 
 // Rows between seeds of the FP64 form.  The FP64 recurrence drifts by
 // ~2^-53 per row, so seeds only bound the work lost to them: 32 m rows keep
@@ -791,19 +803,17 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                          a->max_matches_per_column <= knn_mixed_max_k();
   // Both in double: the exact form (the FP32 band kernel with deterministic
   // bounds, every cell not ruled out in FP64), the matrix under the mixed
-  // form's condition, the lists where each window sees bands enough for a
-  // bound of its k-th best (2 k of them); else the visit kernel.  20011
-  // samples, m = 128, k = 5 above 0.5: visit kernel 6.3 ms; 30000 samples, m =
-  // 100, 50 x 50 entries: 6.9 ms.
+  // form's condition; else the visit kernel.  20011 samples, m = 128, k = 5
+  // above 0.5: visit kernel 6.3 ms, exact form 0.9; 30000 samples, m = 100,
+  // 50 x 50 entries: 6.9 and 0.7 ms; 2000 samples, m = 32: five best 1.25 and
+  // 0.53 ms, one 0.23 and 0.22.
   const bool fp64_exact = a->precision_type == SCAMP_PRECISION_DOUBLE && !nested &&
                           plan.m <= kExactMaxWindow;
   const bool mat_exact = is_mat && fp64_exact && mat_rpc >= kMatMixedMinSpan &&
                          mat_cpc >= kMatMixedMinSpan &&
                          std::max(plan.ns_a, plan.ns_b) < (int64_t{1} << 31) &&
                          static_cast<int64_t>(a->matrix_height) * a->matrix_width < (int64_t{1} << 31);
-  const bool knn_exact = is_knn && fp64_exact && a->max_matches_per_column <= knn_mixed_max_k() &&
-                         std::min(plan.ns_a, plan.ns_b) >=
-                             int64_t{2} * mixed_1nn_band_width() * a->max_matches_per_column;
+  const bool knn_exact = is_knn && fp64_exact && a->max_matches_per_column <= knn_mixed_max_k();
   const bool visit = (is_knn && !knn_mixed && !knn_exact) || (is_mat && !mat_mixed && !mat_exact);
   const bool ultra = a->precision_type == SCAMP_PRECISION_ULTRA;
   const int64_t m = plan.m;
@@ -985,7 +995,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   const bool coarse = kind == K_MIXED && !is_mat && !is_knn &&
                       (a->filter_mode == 2 ||
                        (a->filter_mode == 0 && is_1nn && m >= kCoarseFilterMinWindow));
-  const void* kfn = kind == K_VISIT ? reinterpret_cast<const void*>(join_visit_kernel)
+  const auto visit_fn = is_mat ? join_visit_mat_kernel : join_visit_kernel;
+  const void* kfn = kind == K_VISIT ? reinterpret_cast<const void*>(visit_fn)
                   : kind == K_FP64 ? reinterpret_cast<const void*>(join_fp64_kernel)
                   : mat_exact ? reinterpret_cast<const void*>(join_exact_mat_kernel)
                   : kind == K_EXACT ? reinterpret_cast<const void*>(join_exact_1nn_kernel)
@@ -1142,10 +1153,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       CUDA_TRY(cudaMemsetAsync(q, 0, static_cast<size_t>(P.total_units), st));
       P.fp64_count = dcount + 8;
       P.range = range;
-      // (lists: their k-th bests rise too late to rule many out, so no more
-      // than cost half of what the unit costs the visit kernel)
-      P.req_budget = static_cast<unsigned>(is_knn ? 2 * K * W * 2 / std::max<int64_t>(m, 8)
-                                                  : 2 * K * W / kReqPerCells);
+      // (lists: list_reqs)
+      P.req_budget = is_knn ? UINT32_MAX : static_cast<unsigned>(2 * K * W / kReqPerCells);
       P.wide_budget = static_cast<unsigned>(2 * K * W / kWidePerCells);
     }
     if (band) {
@@ -1154,7 +1163,12 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       // (k-best lists: a window keeps k candidates open, and cold lists
       // ask for more)
       int64_t want = std::max<int64_t>(kMinVerifyReqs, 32 * (nsz[0] + nsz[1]) *
-                                                           (knn_mixed ? 4 * knn_k : 1));
+                                                           (knn_mixed || knn_exact ? 4 * knn_k : 1));
+      const int64_t worth = knn_exact
+          ? static_cast<int64_t>(list_reqs(knn_k) * cells_d / static_cast<double>(m)) + 256 * resident
+          : INT64_MAX;
+      if (knn_exact)
+        want = std::min<int64_t>(want, std::min<int64_t>(kMaxListReqs, std::max(kMinVerifyReqs, worth)));
       want = std::max<int64_t>(want, ws.vreq_seen + ws.vreq_seen / 4);
       want = std::max<int64_t>(std::min<int64_t>(want, kMaxVerifyReqs), ws.vreq_cap);
       void* q;
@@ -1162,7 +1176,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
         return rc;
       ws.vreq_cap = want;
       P.vreq = static_cast<VerifyReq*>(q);
-      P.vreq_cap = want;
+      P.vreq_cap = std::min<int64_t>(want, worth);
     }
     const int64_t grid = std::min<int64_t>(resident, P.total_units);
     if (!nested) {
@@ -1211,6 +1225,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       V.topk[0] = vkeys[0];
       V.topk[1] = vkeys[1];
       V.k = static_cast<int>(knn_k);
+      for (int s = 0; s < 2 && knn_exact; ++s)
+        if (vkeys[s]) V.floor[s] = static_cast<const uint64_t*>(ws.bufs[s ? S_KEY_B : S_KEY_A].p);
       V.mat = vmat;
       V.mat_w = a->matrix_width;
       // grid rows: windows of B (of A in a self-join), columns: windows of A
@@ -1341,12 +1357,12 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       if (is_1nn)
         join_fp64_kernel<<<static_cast<unsigned>(ws.sms * ws.fp64_occ), fp64_threads(), 0, st>>>(F);
       else
-        join_visit_kernel<<<static_cast<unsigned>(ws.sms * ws.visit_occ), visit_threads(), 0, st>>>(
+        visit_fn<<<static_cast<unsigned>(ws.sms * ws.visit_occ), visit_threads(), 0, st>>>(
             F, visit_args());
       verify_exact_kernel<<<static_cast<unsigned>(ws.sms * 8), 256, 0, st>>>(F);
       launches += 2;
     } else if (kind == K_VISIT) {
-      join_visit_kernel<<<static_cast<unsigned>(grid), nthreads, 0, st>>>(P, visit_args());
+      visit_fn<<<static_cast<unsigned>(grid), nthreads, 0, st>>>(P, visit_args());
       ++launches;
     } else {
       join_fp64_kernel<<<static_cast<unsigned>(grid), nthreads, 0, st>>>(P);

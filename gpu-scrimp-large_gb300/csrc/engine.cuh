@@ -244,6 +244,7 @@ struct VisitArgs {
   int mode;                        // 0: k best matches per window, 1: matrix summary
   unsigned long long* topk[2];     // k keys per window of A / B, largest first
   int k;
+  const uint64_t* floor[2];        // lower bounds of the windows' k-th bests, or null
   unsigned* mat;                   // matrix entries (ordered images of floats)
   int64_t mat_w;
   int64_t rows_per_cell, cols_per_cell;
@@ -323,6 +324,7 @@ __global__ void combined_stats_kernel(const double* __restrict__ T, int64_t n, i
                                       double* __restrict__ df, double* __restrict__ dg);
 __global__ void join_fp64_kernel(JoinParams P);
 __global__ void join_visit_kernel(JoinParams P, VisitArgs V);
+__global__ void join_visit_mat_kernel(JoinParams P, VisitArgs V);
 __global__ void floats_to_ord_kernel(const float* __restrict__ in, unsigned* __restrict__ out,
                                      int64_t n);
 __global__ void ord_to_floats_kernel(const unsigned* __restrict__ in, float* __restrict__ out,

@@ -34,7 +34,14 @@ namespace {
 
 constexpr int kVisitThreads = 256;  // one diagonal per thread
 
-__device__ __forceinline__ double seed_dot(const SeriesDev& R, const SeriesDev& C,
+// A diagonal is seeded again where the largest covariance since its seed is
+// ~2^22 times the product of the cell's norms: the recurrence carries that
+// covariance's rounding (two spikes of 1e6 over unit noise, m = 16: r off by
+// 1.5e-6 once they have passed).  Integer operations only, the FP64 pipe is
+// the kernel's bound; anything but such series never seeds again.
+constexpr int kReseed = 22;
+
+__device__ __noinline__ double seed_dot(const SeriesDev& R, const SeriesDev& C,
                                            int64_t i, int64_t j, int64_t m) {
   const double mr = R.mean[i], mc = C.mean[j];
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
@@ -79,13 +86,8 @@ struct CellMax {
   }
 };
 
-}  // namespace
-
-int visit_band_width() { return kVisitThreads; }
-int visit_threads() { return kVisitThreads; }
-
-__global__ void __launch_bounds__(kVisitThreads)
-join_visit_kernel(JoinParams P, VisitArgs V) {
+template <bool kMat>
+__device__ __forceinline__ void visit_body(const JoinParams& P, const VisitArgs& V) {
   __shared__ long long s_unit;
   const int t = threadIdx.x;
   const double thr = P.threshold;
@@ -110,6 +112,8 @@ join_visit_kernel(JoinParams P, VisitArgs V) {
     if (d >= pr.d_hi || (d >= pr.x_lo && d < pr.x_hi)) continue;
     const int64_t rows_b = band_rows(pr.R.ns, pr.C.ns, D0);
     const int ct = V.col_target[pi], rt = V.row_target[pi];
+    const uint64_t* fc = ct >= 0 ? V.floor[ct] : nullptr;
+    const uint64_t* fr = rt >= 0 ? V.floor[rt] : nullptr;
     for (int g = 0; g < 2; ++g) {
       const int64_t i0 = (2 * ub + g) * K;
       int64_t i1 = i0 + K;
@@ -117,6 +121,7 @@ join_visit_kernel(JoinParams P, VisitArgs V) {
       if (i1 > pr.C.ns - d) i1 = pr.C.ns - d;  // this diagonal's last row
       if (i0 >= i1) continue;
       double cov = seed_dot(pr.R, pr.C, i0, i0 + d, P.m);
+      int top = 0;  // high word of the largest |cov| since the seed
       CellMax mc, mr;
       // grid coordinates of the cell, kept by counting: (i / rpc, j / cpc)
       // for column results, (j / rpc, i / cpc) for row results
@@ -124,19 +129,32 @@ join_visit_kernel(JoinParams P, VisitArgs V) {
       Walk wj_r(i0 + d, V.rows_per_cell), wi_c(i0, V.cols_per_cell);
       for (int64_t i = i0; i < i1; ++i) {
         const int64_t j = i + d;
-        const double r = cov * pr.C.inv[j] * pr.R.inv[i];
+        const double inv_c = pr.C.inv[j], inv_r = pr.R.inv[i];
+        double r = cov * inv_c * inv_r;
+        const int mag = __double2hiint(cov) & 0x7fffffff;
+        top = max(top, mag);
+        if ((top >> 20) + (__double2hiint(inv_c) >> 20) + (__double2hiint(inv_r) >> 20) >
+                3 * 1023 + kReseed && r == r) {
+          cov = seed_dot(pr.R, pr.C, i, j, P.m);
+          r = cov * inv_c * inv_r;
+          top = __double2hiint(cov) & 0x7fffffff;
+        }
         if (r > thr) {  // false for NaN (windows that cannot match)
-          if (V.mode == 0) {
+          if constexpr (!kMat) {
+            // (k-th bests from L2: an old value from L1 lets cells insert that
+            // no longer can, 8.3 ms against 5.8 at 20011 samples)
             const uint64_t q = q_from_double_bits(__double_as_longlong(r), P.kl.frac_bits);
             if (ct >= 0) {
               unsigned long long* sl = V.topk[ct] + j * V.k;
               const unsigned long long key = make_key(q, i, P.kl);
-              if (key > sl[V.k - 1]) topk_insert(sl, V.k, key);
+              if (key > __ldcg(sl + V.k - 1) && (!fc || q >= fc[j] >> P.kl.idx_bits))
+                topk_insert(sl, V.k, key);
             }
             if (rt >= 0) {
               unsigned long long* sl = V.topk[rt] + i * V.k;
               const unsigned long long key = make_key(q, j, P.kl);
-              if (key > sl[V.k - 1]) topk_insert(sl, V.k, key);
+              if (key > __ldcg(sl + V.k - 1) && (!fr || q >= fr[i] >> P.kl.idx_bits))
+                topk_insert(sl, V.k, key);
             }
           } else {
             // grid rows are windows of B, columns windows of A; a target of
@@ -148,19 +166,38 @@ join_visit_kernel(JoinParams P, VisitArgs V) {
         }
         cov = fma(pr.C.df[j], pr.R.dg[i], cov);
         cov = fma(pr.R.df[i], pr.C.dg[j], cov);
-        if (V.mode == 1) {
+        if constexpr (kMat) {
           wi_r.next();
           wj_c.next();
           wj_r.next();
           wi_c.next();
         }
       }
-      if (V.mode == 1) {
+      if constexpr (kMat) {
         mc.flush(V.mat);
         mr.flush(V.mat);
       }
     }
   }
+}
+
+}  // namespace
+
+int visit_band_width() { return kVisitThreads; }
+int visit_threads() { return kVisitThreads; }
+
+// Lists: latency of the insertions, so four CTAs per SM rather than registers
+// (20011 samples, m = 128, five best above 0.5: two CTAs 9.8 ms, four 5.5).
+__global__ void __launch_bounds__(kVisitThreads, 4)
+join_visit_kernel(JoinParams P, VisitArgs V) {
+  visit_body<false>(P, V);
+}
+
+// Grid: the walk itself, so registers (117 of them and two CTAs per SM; as one
+// kernel with the lists, 64 registers, 4.3 ms for the same samples, now 3.55).
+__global__ void __launch_bounds__(kVisitThreads)
+join_visit_mat_kernel(JoinParams P, VisitArgs V) {
+  visit_body<true>(P, V);
 }
 
 // Matrix entries between floats (-2 = none) and their ordered images.

@@ -2,9 +2,9 @@
 the FP32 filter, against brute-force correlation matrices.
 
 The filter may only skip cells that its bounds rule out, so lists and grids
-must be the FP64 ones.  Lists take it from 2048 k windows on, grids from
-entries of 64 windows on; sizes sit at those edges and at the edges of its
-1024-diagonal bands.  Tolerance as in the brute-force checks it reuses:
+must be the FP64 ones.  Lists take it at every size, grids from entries of
+64 windows on; sizes sit at that edge, at the edges of its 1024-diagonal
+bands, and where a window has fewer bands or cells than its list entries.  Tolerance as in the brute-force checks it reuses:
 float32 rounding of an FP64 correlation.
 """
 import numpy as np
@@ -43,6 +43,28 @@ def test_lists(gpu_engine, kind, n, nb, m, k, thr):
     r = gpu_engine.join(a, b, m, "ALL_NEIGHBORS", "double", threshold=thr, max_matches=k,
                         keep_rows=nb is not None)
     assert r["counters"]["steps"] > 0  # the filter ran
+    C = self_matrix(a, m) if b is None else corr_matrix(b, a, m)
+    check_knn(gpu_engine, r["knn_a"], k, C, thr, kind + "/A")
+    if b is not None:
+        check_knn(gpu_engine, r["knn_b"], k, C.T, thr, kind + "/B")
+
+
+@pytest.mark.parametrize("kind", ["walk", "gaps", "spikes", "square"])
+@pytest.mark.parametrize("n,nb,m,k,thr", [(300, None, 16, 64, 0.0), (1100, 330, 30, 7, 0.2),
+                                          (1023 + 32, None, 32, 64, -1.0), (2600, None, 50, 20, 0.4)])
+def test_short_lists(gpu_engine, kind, n, nb, m, k, thr):
+    """Fewer bands than list entries, lists longer than a window has cells,
+    exact repeats (no bound separates their cells)."""
+    def make(length, seed):
+        if kind == "square":
+            return (np.arange(length) // 7 % 2).astype(float)
+        return series(kind, length, seed)
+
+    a = make(n, 4)
+    b = None if nb is None else make(nb, 5)
+    r = gpu_engine.join(a, b, m, "ALL_NEIGHBORS", "double", threshold=thr, max_matches=k,
+                        keep_rows=nb is not None)
+    assert r["counters"]["steps"] > 0
     C = self_matrix(a, m) if b is None else corr_matrix(b, a, m)
     check_knn(gpu_engine, r["knn_a"], k, C, thr, kind + "/A")
     if b is not None:
