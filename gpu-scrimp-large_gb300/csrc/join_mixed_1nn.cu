@@ -201,6 +201,7 @@ struct SlowItem {
 // CTA-uniform context of the exact path, kept in shared memory.
 struct SlowCtx {
   const Problem* pr;
+  uint64_t *key_row, *key_col;  // the problem's
   int64_t rbase[2];
   int64_t D0;  // first diagonal of the unit; thread t owns D0 + t*kDiags ..
   int ring0;   // ring column of the slab's first staged column
@@ -438,18 +439,17 @@ __device__ __noinline__ float verify_cov_lane(const SeriesDev& R, const SeriesDe
 
 __device__ __forceinline__ void publish(Smem& sm, const SlowCtx& cx, float rv, int64_t i,
                                         int64_t j, int rslot, int cslot, int g) {
-  const Problem& pr = *cx.pr;
   const float rb = g ? sm.r_best[rslot].y : sm.r_best[rslot].x;
   const float cb = g ? sm.c_best[padc(cslot)].y : sm.c_best[padc(cslot)].x;
   if (rv > rb) {
-    atomicMax(reinterpret_cast<u64*>(pr.key_row + i),
+    atomicMax(reinterpret_cast<u64*>(cx.key_row + i),
               make_key(q_from_float_bits(__float_as_uint(rv), cx.kl.frac_bits), j, cx.kl));
     // The float copies only filter candidates; a racing store of a smaller
     // value costs extra work later, never a wrong result.
     if (g) sm.r_best[rslot].y = rv; else sm.r_best[rslot].x = rv;
   }
   if (rv > cb) {
-    atomicMax(reinterpret_cast<u64*>(pr.key_col + j),
+    atomicMax(reinterpret_cast<u64*>(cx.key_col + j),
               make_key(q_from_float_bits(__float_as_uint(rv), cx.kl.frac_bits), i, cx.kl));
     if (g) sm.c_best[padc(cslot)].y = rv; else sm.c_best[padc(cslot)].x = rv;
   }
@@ -537,16 +537,17 @@ __device__ __forceinline__ void close_requests(Smem& sm, const SlowCtx& cx, int 
 // n consecutive slots of the request buffer for the warp, from a block of
 // kReqChunk that it takes at a time, so that the global counter's round trip
 // is paid once per block and not once per row of candidates.  Called by the
-// whole warp, n <= kReqChunk.
+// whole warp; more than a block's slots come as whole blocks.
 __device__ __forceinline__ unsigned long long take_requests(Smem& sm, const SlowCtx& cx, int warp,
                                                             int lane, int n) {
   int used = sm.rq_used[warp];
   unsigned long long base = sm.rq_base[warp];
   if (used + n > kReqChunk) {
     close_requests(sm, cx, warp, lane);
-    if (lane == 0) base = atomicAdd(cx.vcount, static_cast<unsigned long long>(kReqChunk));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    used = 0;
+    const int whole = (n - 1) / kReqChunk * kReqChunk;  // slots before the last block
+    if (lane == 0) base = atomicAdd(cx.vcount, static_cast<unsigned long long>(whole + kReqChunk));
+    base = __shfl_sync(0xffffffffu, base, 0) + whole;
+    used = -whole;
   }
   __syncwarp();
   if (lane == 0) {
@@ -555,6 +556,16 @@ __device__ __forceinline__ unsigned long long take_requests(Smem& sm, const Slow
   }
   __syncwarp();
   return base + used;
+}
+
+// Sum of v over the lanes up to this one.
+__device__ __forceinline__ int warp_prefix(int v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int w = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += w;
+  }
+  return v;
 }
 
 // Exact path of queued blocks, 8 lanes per block (four blocks per pass):
@@ -733,6 +744,16 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
   return nreq;
 }
 
+// Exact form: counts n requests, `wide` of them of wide bounds and the last
+// below slot `end`, against what the unit may make.
+__device__ __forceinline__ void spend_requests(Smem& sm, const SlowCtx& cx, unsigned n,
+                                               unsigned wide, unsigned long long end) {
+  if (atomicAdd(&sm.cx.unit_reqs, n) + n > cx.budget ||
+      (wide && atomicAdd(&sm.cx.unit_wide, wide) + wide > cx.wide_budget) ||
+      end > static_cast<unsigned long long>(cx.vcap))
+    sm.cx.unit_lost = 1;
+}
+
 // Exact form: writes the requests of the lanes that qx, qy mark (segments x
 // and y of cells (i, i + d)).  Called by the whole warp; returns the number
 // written.
@@ -760,11 +781,7 @@ __device__ __forceinline__ int push_requests(Smem& sm, const SlowCtx& cx, int wa
   }
   const unsigned wide = __popc(__ballot_sync(0xffffffffu, qx && mk.x > kWideBound)) +
                         __popc(__ballot_sync(0xffffffffu, qy && mk.y > kWideBound));
-  if (lane == 0 &&
-      (atomicAdd(&sm.cx.unit_reqs, static_cast<unsigned>(n)) + n > cx.budget ||
-       (wide && atomicAdd(&sm.cx.unit_wide, wide) + wide > cx.wide_budget) ||
-       base + n > static_cast<unsigned long long>(cx.vcap)))
-    sm.cx.unit_lost = 1;
+  if (lane == 0) spend_requests(sm, cx, static_cast<unsigned>(n), wide, base + n);
   __syncwarp();
   return n;
 }
@@ -774,17 +791,16 @@ __device__ __forceinline__ int push_requests(Smem& sm, const SlowCtx& cx, int wa
 // racing store of a smaller value costs extra work, never a wrong result).
 __device__ __forceinline__ void publish_bound(Smem& sm, const SlowCtx& cx, float lb, int64_t i,
                                               int64_t j, int rslot, int cslot, int g) {
-  const Problem& pr = *cx.pr;
   if (!(lb > -2.f)) return;
   float& rb = g ? sm.r_best[rslot].y : sm.r_best[rslot].x;
   float& cb = g ? sm.c_best[padc(cslot)].y : sm.c_best[padc(cslot)].x;
   const uint64_t q = q_from_float_bits(__float_as_uint(lb), cx.kl.frac_bits);
   if (lb > rb) {
-    atomicMax(reinterpret_cast<u64*>(pr.key_row + i), make_key(q, j, cx.kl));
+    atomicMax(reinterpret_cast<u64*>(cx.key_row + i), make_key(q, j, cx.kl));
     rb = lb;
   }
   if (lb > cb) {
-    atomicMax(reinterpret_cast<u64*>(pr.key_col + j), make_key(q, i, cx.kl));
+    atomicMax(reinterpret_cast<u64*>(cx.key_col + j), make_key(q, i, cx.kl));
     cb = lb;
   }
 }
@@ -818,13 +834,16 @@ __device__ __forceinline__ float mat_cell_floor(const SlowCtx& cx, int64_t i, in
 template <bool kMat>
 __device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane) {
   __syncwarp();  // the queue was written by other lanes
-  const SlowCtx& cx = sm.cx;
-  // a unit left to the FP64 kernel needs no more requests (lane 0's view:
-  // another warp may be setting it)
-  if (__shfl_sync(0xffffffffu, *const_cast<volatile unsigned*>(&sm.cx.unit_lost), 0)) return 0;
+  // (in registers: read again after every store otherwise; m = 1024 with gaps
+  // 2.89 -> 2.75 ms.  The mixed form's exact path has no registers left for
+  // it: its kernels spilled, 9% slower.)
+  const SlowCtx cx = sm.cx;
   const int k = lane & 7;
   int nreq = 0;
   for (int p = 0; p < count; p += 4) {
+    // a unit left to the FP64 kernel needs no more requests (lane 0's view:
+    // another warp may be setting it)
+    if (__shfl_sync(0xffffffffu, *const_cast<volatile unsigned*>(&sm.cx.unit_lost), 0)) break;
     const int item = p + (lane >> 3);
     const bool act = item < count;
     const SlowItem& it = sm.queue[warp][act ? item : 0];
@@ -836,42 +855,106 @@ __device__ __noinline__ int drain_exact(Smem& sm, int warp, int count, int lane)
     const int r0 = s0 * kRows;
     const int cb0 = 8 * (s0 + it.owner) + k;           // staged column at row 0
     const int64_t jd = cx.D0 + it.owner * kDiags + k;  // the lane's diagonal
+    if constexpr (!kMat) {
+      // A step's rows are first all filtered, their loads in flight together;
+      // then one reservation holds every candidate's request, and each lane
+      // writes and publishes its own (those that the bests raised meanwhile
+      // rule out as requests that rule themselves out).  Row by row, a row
+      // with candidates was ~1300 cycles of one warp's latency: band kernels
+      // and verification of 40009 samples with gaps, m = 1024, 2.87 -> 2.52 ms,
+      // 60000 x 30011, m = 256, 1.25 -> 1.16, 1000, m = 50, 0.130 -> 0.118.
 #pragma unroll 1
-    for (int rw = nrows_w - 1; rw >= 0; --rw) {
-      const bool live = rw < nrows;
-      const int rr = live ? rw : 0;  // rows past the block's end read row 0
-      const int rcs = ringc(cx.ring0, cb0 + rr);
-      const float4 rf = sm.r_fg[r0 + rr];
-      const float4 cf = col_fg(sm, padc(rcs));
-      if (live) {
-        c = fma2(make_float2(-rf.x, -rf.y), make_float2(cf.z, cf.w), c);
-        c = fma2(make_float2(-cf.x, -cf.y), make_float2(rf.z, rf.w), c);
+      for (int b = nrows_w / kRows - 1; b >= 0; --b) {
+        const bool live = b * kRows < nrows;
+        const int q0 = live ? b * kRows : 0;  // a step past the block's end reads its first
+        float2 rvs[kRows];
+        unsigned cand = 0;  // bit u: row u of the first segment, bit u + 8: of the second
+#pragma unroll
+        for (int u = kRows - 1; u >= 0; --u) {
+          const int rr = q0 + u;
+          const int slot = padc(ringc(cx.ring0, cb0 + rr));
+          const float4 rf = sm.r_fg[r0 + rr];
+          const float4 cf = col_fg(sm, slot);
+          if (live) {
+            c = fma2(make_float2(-rf.x, -rf.y), make_float2(cf.z, cf.w), c);
+            c = fma2(make_float2(-cf.x, -cf.y), make_float2(rf.z, rf.w), c);
+          }
+          const float2 ivr = sm.r_iv[r0 + rr];
+          const float2 ivc = sm.u.s.c_iv[slot];
+          const float2 rv = mul2(mul2(c, ivc), ivr);
+          const float2 mk = mul2(mul2(vw, ivc), ivr);
+          const float2 rb = sm.r_best[r0 + rr];
+          const float2 cbv = sm.c_best[slot];
+          // (false for NaN: excluded diagonals, windows that cannot match)
+          if (rv.x + (mk.x + kAbsSlack) > fminf(rb.x, cbv.x)) cand |= 1u << u;
+          if (rv.y + (mk.y + kAbsSlack) > fminf(rb.y, cbv.y)) cand |= 256u << u;
+          rvs[u] = rv;
+        }
+        if (!live) cand = 0;
+        const int mine = __popc(cand);
+        const int upto = warp_prefix(mine, lane);
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+        if (total == 0) continue;
+        const unsigned long long base = take_requests(sm, cx, warp, lane, total);
+        unsigned long long slot = base + (upto - mine);
+        unsigned real = 0, wide = 0;
+#pragma unroll 1
+        while (cand) {
+          const int bit = 31 - __clz(cand);
+          cand &= ~(1u << bit);
+          const int u = bit & 7, g = bit >> 3, rr = q0 + u;
+          const int rcs = ringc(cx.ring0, cb0 + rr);
+          const float2 mk2 = mul2(mul2(vw, sm.u.s.c_iv[padc(rcs)]), sm.r_iv[r0 + rr]);
+          const float2 rb = sm.r_best[r0 + rr];
+          const float2 cbv = sm.c_best[padc(rcs)];
+          const float rv = g ? rvs[u].y : rvs[u].x, mk = (g ? mk2.y : mk2.x) + kAbsSlack;
+          const bool ok = rv + mk > (g ? fminf(rb.y, cbv.y) : fminf(rb.x, cbv.x));
+          const int64_t i = cx.rbase[g] + r0 + rr;
+          if (slot < static_cast<unsigned long long>(cx.vcap)) {
+            VerifyReq rq;
+            rq.i = static_cast<uint64_t>(i) | (static_cast<uint64_t>(cx.prob) << 40);
+            rq.d = static_cast<uint32_t>(jd);
+            rq.ub = ok ? rv + mk : -4.f;
+            cx.vreq[slot] = rq;
+          }
+          ++slot;
+          if (!ok) continue;
+          ++real;
+          wide += mk > kWideBound ? 1u : 0u;
+          // (one cell's bound says nothing of a window's k-th best)
+          if (!cx.knn_k) publish_bound(sm, cx, rv - mk, i, i + jd, r0 + rr, rcs, g);
+        }
+        __syncwarp();
+        real = __reduce_add_sync(0xffffffffu, real);
+        wide = __reduce_add_sync(0xffffffffu, wide);
+        nreq += static_cast<int>(real);
+        if (lane == 0) spend_requests(sm, cx, real, wide, base + total);
       }
-      const float2 ivr = sm.r_iv[r0 + rr];
-      const float2 ivc = sm.u.s.c_iv[padc(rcs)];
-      const float2 rv = mul2(mul2(c, ivc), ivr);
-      const float2 mk0 = mul2(mul2(vw, ivc), ivr);
-      const float2 mk = make_float2(mk0.x + kAbsSlack, mk0.y + kAbsSlack);
-      const int64_t i0 = cx.rbase[0] + r0 + rr, i1 = cx.rbase[1] + r0 + rr;
-      // (false for NaN: excluded diagonals, windows that cannot match)
-      bool cx_, cy_;
-      if constexpr (kMat) {
-        cx_ = live && rv.x + mk.x > cx.thr;
-        cy_ = live && rv.y + mk.y > cx.thr;
+    } else {
+      // matrix: most rows hold a candidate of some grid entry's floor test
+#pragma unroll 1
+      for (int rw = nrows_w - 1; rw >= 0; --rw) {
+        const bool live = rw < nrows;
+        const int rr = live ? rw : 0;  // rows past the block's end read row 0
+        const int slot = padc(ringc(cx.ring0, cb0 + rr));
+        const float4 rf = sm.r_fg[r0 + rr];
+        const float4 cf = col_fg(sm, slot);
+        if (live) {
+          c = fma2(make_float2(-rf.x, -rf.y), make_float2(cf.z, cf.w), c);
+          c = fma2(make_float2(-cf.x, -cf.y), make_float2(rf.z, rf.w), c);
+        }
+        const float2 ivr = sm.r_iv[r0 + rr];
+        const float2 ivc = sm.u.s.c_iv[slot];
+        const float2 rv = mul2(mul2(c, ivc), ivr);
+        const float2 mk0 = mul2(mul2(vw, ivc), ivr);
+        const float2 mk = make_float2(mk0.x + kAbsSlack, mk0.y + kAbsSlack);
+        const int64_t i0 = cx.rbase[0] + r0 + rr, i1 = cx.rbase[1] + r0 + rr;
+        // (false for NaN: excluded diagonals, windows that cannot match)
+        bool cx_ = live && rv.x + mk.x > cx.thr, cy_ = live && rv.y + mk.y > cx.thr;
         if (cx_) cx_ = rv.x + mk.x > mat_cell_floor(cx, i0, i0 + jd);
         if (cy_) cy_ = rv.y + mk.y > mat_cell_floor(cx, i1, i1 + jd);
-      } else {
-        const float2 rb = sm.r_best[r0 + rr];
-        const float2 cbv = sm.c_best[padc(rcs)];
-        cx_ = live && rv.x + mk.x > fminf(rb.x, cbv.x);
-        cy_ = live && rv.y + mk.y > fminf(rb.y, cbv.y);
+        nreq += push_requests(sm, cx, warp, lane, cx_, cy_, rv, mk, i0, i1, jd);
       }
-      if (!__any_sync(0xffffffffu, cx_ || cy_)) continue;
-      nreq += push_requests(sm, cx, warp, lane, cx_, cy_, rv, mk, i0, i1, jd);
-      // (one cell's bound says nothing of a window's k-th best)
-      if (kMat || cx.knn_k) continue;
-      if (cx_) publish_bound(sm, cx, rv.x - mk.x, i0, i0 + jd, r0 + rr, rcs, 0);
-      if (cy_) publish_bound(sm, cx, rv.y - mk.y, i1, i1 + jd, r0 + rr, rcs, 1);
     }
   }
   __syncwarp();
@@ -1420,6 +1503,8 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
       // read by the exact path only after the slab's first barrier
       SlowCtx& cx = sm.cx;
       cx.pr = &sm.prob;
+      cx.key_row = pr.key_row;
+      cx.key_col = pr.key_col;
       cx.D0 = D0;
       cx.m = m;
       cx.kl = P.kl;
