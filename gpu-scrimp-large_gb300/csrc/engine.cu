@@ -153,6 +153,15 @@ int64_t exact_segment(double cells, int64_t resident, int W, int slab, int64_t m
 // a flat stretch leaves FP32 nothing, so a few say that the unit is lost.
 constexpr int64_t kReqPerCells = 4;
 constexpr int64_t kWidePerCells = 1024;
+// Requests of a 1NN join of the exact form in all, per cell over the window
+// length: where exact repeats everywhere leave every bound open, verifying
+// costs more than the FP64 band kernel, which then takes the units beyond
+// this.  60000 samples of a square wave, m = 1000: 197 ms without a limit, 26.8
+// with it, FP64 band kernel alone 45; near-ties stay worth verifying (30000
+// samples of a sine, m = 1024, 3.2 requests per cell over m: 7.7 ms, with a limit
+// of 2 10.1, of 1 12.9); random walks make 1.0 and fewer.
+constexpr double kExactReqs = 4.0;
+
 // Requests of a k-best join in all, per cell over the window length; the units
 // beyond them are left to the visit kernel, whose time grows with k.  No
 // budget per unit: a unit of dense matches, one insertion after the other,
@@ -1164,8 +1173,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       // ask for more)
       int64_t want = std::max<int64_t>(kMinVerifyReqs, 32 * (nsz[0] + nsz[1]) *
                                                            (knn_mixed || knn_exact ? 4 * knn_k : 1));
-      const int64_t worth = knn_exact
-          ? static_cast<int64_t>(list_reqs(knn_k) * cells_d / static_cast<double>(m)) + 256 * resident
+      const double per_cell = knn_exact ? list_reqs(knn_k)
+                            : kind == K_EXACT && is_1nn ? kExactReqs : 0.0;
+      const int64_t worth = per_cell > 0.0
+          ? static_cast<int64_t>(per_cell * cells_d / static_cast<double>(m)) + 256 * resident
           : INT64_MAX;
       if (knn_exact)
         want = std::min<int64_t>(want, std::min<int64_t>(kMaxListReqs, std::max(kMinVerifyReqs, worth)));

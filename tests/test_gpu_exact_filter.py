@@ -57,3 +57,14 @@ def test_double_profile(gpu_engine, oracle_mod, kind, n, nb, m):
     if nb is not None:
         _, gi = gpu_engine.unpack_profile(got["profile_b"])
         check_1nn_direct(kind + "/B", got["corr_b"], gi, want["idx_b"], TOL_FP64, b, a, m)
+
+
+@pytest.mark.parametrize("n,m", [(12000, 700), (9000, 1500)])
+def test_more_requests_than_worth_verifying(gpu_engine, oracle_mod, n, m):
+    """Exact repeats of every window: the join's limit of requests leaves
+    units to the FP64 band kernel midway, whose requests must be void."""
+    a = (np.arange(n) // 25 % 2).astype(float)
+    got = gpu_engine.join(a, None, m, precision="double", return_corr=True)
+    want = oracle_mod.join(a, None, m, "1NN_INDEX", exact_flat=True)
+    _, gi = gpu_engine.unpack_profile(got["profile_a"])
+    check_1nn_direct("square", got["corr_a"], gi, want["idx_a"], TOL_FP64, a, a, m)
