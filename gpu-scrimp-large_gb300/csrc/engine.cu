@@ -172,6 +172,11 @@ constexpr double kExactReqs = 4.0;
 // bound separates the best cells (60000 samples of a square wave, m = 1000,
 // five best) all requests would take 195 ms, the visit kernel takes 43, this
 // both in part: 46.
+// A visited unit of dense matches takes 2 ms whatever the join's size, which
+// is kListReqsLatency / m requests' time (~4.3 ps x m each): 2419 samples with
+// gaps, m = 117, ten best, half of the series 2.2-2.8 ms at 390000 requests,
+// now all 0.7.
+constexpr int64_t kListReqsLatency = int64_t{1} << 29;
 double list_reqs(int64_t k) { return 3.0 + 0.75 * static_cast<double>(k); }
 constexpr int64_t kMaxListReqs = int64_t{1} << 27;  // 2 GiB of requests
 
@@ -1176,7 +1181,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       const double per_cell = knn_exact ? list_reqs(knn_k)
                             : kind == K_EXACT && is_1nn ? kExactReqs : 0.0;
       const int64_t worth = per_cell > 0.0
-          ? static_cast<int64_t>(per_cell * cells_d / static_cast<double>(m)) + 256 * resident
+          ? static_cast<int64_t>(per_cell * cells_d / static_cast<double>(m)) +
+                (knn_exact ? kListReqsLatency / m : 256 * resident)
           : INT64_MAX;
       if (knn_exact)
         want = std::min<int64_t>(want, std::min<int64_t>(kMaxListReqs, std::max(kMinVerifyReqs, worth)));
