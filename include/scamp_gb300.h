@@ -119,7 +119,8 @@ typedef struct scamp_c_result {
                          * a direct dot product inside the band kernel because
                          * the request buffer was full (slow; the next join on
                          * the device sizes the buffer for them); saturates */
-  /* Work counters of the mixed 1NN_INDEX form (0 otherwise): 8-row steps
+  /* Work counters of the mixed forms and of DOUBLE joins behind the FP32
+   * filter (0 otherwise): 8-row steps
    * of one thread, steps recomputed on the exact path, and candidate cells
    * sent to verification by a direct dot product. */
   uint64_t steps;
