@@ -137,12 +137,21 @@ constexpr int64_t kExactMaxWindow = 65536;
 // its anchors and about 3 per cell, and the last wave is half empty, so the
 // time goes as (v + 1/2) (m + 3 K_1 / v), K_1 the rows of one wave's units:
 // least at v = sqrt(3 K_1 / 2 m).  Whole slabs, or a fraction of one where
-// the join has fewer units than resident CTAs.
+// the join has fewer units than resident CTAs.  A unit also costs its first
+// slab's full staging (1152 columns, 128 from then on), which decides where
+// a wave is three slabs or less: one wave then (band kernels: 20000 samples,
+// m = 100, 128 rows 0.33 ms, 256 0.29; 30000, m = 300, 128 0.76, 384 0.58; m =
+// 1000 1.65 and 1.23; but 33324, m = 76, 512 rows, one wave, 9% slower than
+// 256), and below m = 128 at least four slabs in joins of six and more
+// (45000, m = 100, 256 rows 0.77, 512 0.71; 60000, m = 64, 1.09 and 1.00; m =
+// 278 5% slower).
 int64_t exact_segment(double cells, int64_t resident, int W, int slab, int64_t m) {
   const double k1 = cells / (2.0 * W * static_cast<double>(resident));
   if (k1 < slab) return (static_cast<int64_t>(k1) / 32 + 1) * 32;
+  if (k1 < 3 * slab) return (static_cast<int64_t>(k1) / slab + 1) * slab;
   const double v = std::min(8.0, std::max(3.0, std::sqrt(1.5 * k1 / static_cast<double>(m))));
-  return (static_cast<int64_t>(k1 / v) / slab + 1) * slab;
+  const int64_t k = (static_cast<int64_t>(k1 / v) / slab + 1) * slab;
+  return m < 128 && k1 >= 6 * slab ? std::max<int64_t>(k, 4 * slab) : k;
 }
 
 // Verification requests a unit of the exact form may make before the FP64
