@@ -622,8 +622,33 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
     // covariance the fast path used in row rr (the order of a block's rows
     // does not matter: updates are atomic maxima or sums, and every floor
     // read is a value already published)
-    // one row: the lanes' cells that may improve its or their column's best
-    auto settle = [&](int rr, int rcs, float2 rv, float2 mk, bool cx_, bool cy_, float tx, float ty) {
+#pragma unroll 1
+    for (int rw = kMerged ? nrows_w - 1 : 0; kMerged ? rw >= 0 : rw < nrows_w;
+         rw += kMerged ? -1 : 1) {
+      const bool live = rw < nrows;
+      const int rr = live ? rw : 0;  // rows past the block's end read row 0
+      const int cs = cb0 + rr;
+      const int rcs = ringc(cx.ring0, cs);  // its ring column
+      const float4 rf = sm.r_fg[r0 + rr];
+      const float4 cf = col_fg(sm, padc(rcs));
+      if constexpr (kMerged) {
+        if (live) {
+          c = fma2(make_float2(-rf.x, -rf.y), make_float2(cf.z, cf.w), c);
+          c = fma2(make_float2(-cf.x, -cf.y), make_float2(rf.z, rf.w), c);
+        }
+      }
+      const float2 ivr = sm.r_iv[r0 + rr];
+      const float2 ivc = sm.u.s.c_iv[padc(rcs)];
+      const float2 rv = mul2(mul2(c, ivc), ivr);  // the fast path's rounding
+      const float2 mk = mul2(mul2(vk, ivc), ivr);
+      const float2 rb = sm.r_best[r0 + rr];
+      const float2 cbv = sm.c_best[padc(rcs)];
+      // the value to beat: the row's and column's bests, or the threshold
+      const float tx = cx.sum_mode ? cx.thr : fminf(rb.x, cbv.x);
+      const float ty = cx.sum_mode ? cx.thr : fminf(rb.y, cbv.y);
+      const int sm2 = msk >> (2 * (rw >> 3));
+      const bool cx_ = live && (sm2 & 1) && rv.x + mk.x > tx;
+      const bool cy_ = live && (sm2 & 2) && rv.y + mk.y > ty;
       // SUM_THRESH: a cell surely above the threshold counts with its FP32 r
       const bool qx = cx_ && mk.x > kTrust && !(cx.sum_mode && rv.x - mk.x > tx);
       const bool qy = cy_ && mk.y > kTrust && !(cx.sum_mode && rv.y - mk.y > ty);
@@ -657,81 +682,9 @@ __device__ __noinline__ int drain_queue(Smem& sm, int warp, int count, int lane)
           if (rs.y != 0.f) atomicAdd(&sm.r_best[r0 + rr].y, rs.y);
         }
       }
-    };
-    // the value to beat: the row's and column's bests, or the threshold
-    auto beat = [&](float r, float c) { return cx.sum_mode ? cx.thr : fminf(r, c); };
-    if constexpr (kMerged) {
-#pragma unroll 1
-      for (int rw = nrows_w - 1; rw >= 0; --rw) {
-        const bool live = rw < nrows;
-        const int rr = live ? rw : 0;  // rows past the block's end read row 0
-        const int rcs = ringc(cx.ring0, cb0 + rr);  // its ring column
-        const float4 rf = sm.r_fg[r0 + rr];
-        const float4 cf = col_fg(sm, padc(rcs));
-        if (live) {
-          c = fma2(make_float2(-rf.x, -rf.y), make_float2(cf.z, cf.w), c);
-          c = fma2(make_float2(-cf.x, -cf.y), make_float2(rf.z, rf.w), c);
-        }
-        const float2 ivr = sm.r_iv[r0 + rr];
-        const float2 ivc = sm.u.s.c_iv[padc(rcs)];
-        const float2 rv = mul2(mul2(c, ivc), ivr);  // the fast path's rounding
-        const float2 mk = mul2(mul2(vk, ivc), ivr);
-        const float2 rb = sm.r_best[r0 + rr];
-        const float2 cbv = sm.c_best[padc(rcs)];
-        const float tx = beat(rb.x, cbv.x), ty = beat(rb.y, cbv.y);
-        const int sm2 = msk >> (2 * (rw >> 3));
-        settle(rr, rcs, rv, mk, live && (sm2 & 1) && rv.x + mk.x > tx,
-               live && (sm2 & 2) && rv.y + mk.y > ty, tx, ty);
-      }
-    } else {
-      // A step's rows are first all filtered, their loads and covariances in
-      // flight together, then the rows with candidates are settled one by
-      // one, each against the bests of that moment: the walk is one warp's
-      // latency while the others wait at the slab's end (band kernel, 2^20
-      // windows of m = 1024: 94.7 -> 90.0 ms, 76.7 with no exact path at all;
-      // the one-pass forms gain nothing, batches' hot blocks lost 19%).
-#pragma unroll 1
-      for (int b = 0; b < nrows_w / kRows; ++b) {
-        const bool live = b * kRows < nrows;
-        const int q0 = live ? b * kRows : 0;  // a step past the block's end reads its first
-        const int sm2 = live ? msk >> (2 * b) : 0;
-        float2 rvs[kRows];
-        unsigned cand = 0;  // bit u: row u of the first segment, bit u + 8: of the second
-#pragma unroll
-        for (int u = 0; u < kRows; ++u) {
-          const int rr = q0 + u;
-          const int slot = padc(ringc(cx.ring0, cb0 + rr));
-          const float4 rf = sm.r_fg[r0 + rr];
-          const float4 cf = col_fg(sm, slot);
-          const float2 ivr = sm.r_iv[r0 + rr];
-          const float2 ivc = sm.u.s.c_iv[slot];
-          const float2 rv = mul2(mul2(c, ivc), ivr);  // the fast path's rounding
-          const float2 mk = mul2(mul2(vk, ivc), ivr);
-          const float2 rb = sm.r_best[r0 + rr];
-          const float2 cbv = sm.c_best[slot];
-          if (rv.x + mk.x > beat(rb.x, cbv.x)) cand |= 1u << u;
-          if (rv.y + mk.y > beat(rb.y, cbv.y)) cand |= 256u << u;
-          rvs[u] = rv;
-          c = fma2(make_float2(cf.x, cf.y), make_float2(rf.z, rf.w), c);
-          c = fma2(make_float2(rf.x, rf.y), make_float2(cf.z, cf.w), c);
-        }
-        cand &= ((sm2 & 1) ? 255u : 0u) | ((sm2 & 2) ? 255u << 8 : 0u);
-        unsigned rows = __reduce_or_sync(0xffffffffu, cand);
-        rows = (rows | rows >> 8) & 255u;
-#pragma unroll 1
-        while (rows) {
-          const int u = __ffs(rows) - 1;
-          rows &= rows - 1;
-          const int rr = q0 + u;
-          const int rcs = ringc(cx.ring0, cb0 + rr);
-          const float2 rv = rvs[u];
-          const float2 mk = mul2(mul2(vk, sm.u.s.c_iv[padc(rcs)]), sm.r_iv[r0 + rr]);
-          const float2 rb = sm.r_best[r0 + rr];
-          const float2 cbv = sm.c_best[padc(rcs)];
-          const float tx = beat(rb.x, cbv.x), ty = beat(rb.y, cbv.y);
-          settle(rr, rcs, rv, mk, (cand >> u & 1u) && rv.x + mk.x > tx,
-                 (cand >> u & 256u) && rv.y + mk.y > ty, tx, ty);
-        }
+      if constexpr (!kMerged) {
+        c = fma2(make_float2(cf.x, cf.y), make_float2(rf.z, rf.w), c);
+        c = fma2(make_float2(rf.x, rf.y), make_float2(cf.z, cf.w), c);
       }
     }
   }
