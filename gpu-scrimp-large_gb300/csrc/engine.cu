@@ -549,20 +549,13 @@ void set_keys(JoinParams& P, const Plan& plan, int s, uint64_t* keys) {
   }
 }
 
-// The bounds pass over the units of P (its own queue head).
-int launch_bounds(const JoinParams& P, bool exact, int64_t grid, size_t smem, cudaStream_t st,
-                  std::string* msg) {
-  const void* fn = P.mat ? reinterpret_cast<const void*>(bound_exact_mat_kernel)
-                 : exact ? reinterpret_cast<const void*>(bound_exact_1nn_kernel)
-                         : reinterpret_cast<const void*>(bound_mixed_1nn_kernel);
-  CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+// The exact form's bounds pass over the units of P (its own queue head).
+int launch_bounds(const JoinParams& P, int64_t grid, size_t smem, cudaStream_t st, std::string* msg) {
+  const auto fn = P.mat ? bound_exact_mat_kernel : bound_exact_1nn_kernel;
+  CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem)));
-  if (P.mat)
-    bound_exact_mat_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
-  else if (exact)
-    bound_exact_1nn_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
-  else
-    bound_mixed_1nn_kernel<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
+  fn<<<static_cast<unsigned>(grid), mixed_1nn_threads(), smem, st>>>(P);
   CUDA_TRY(cudaGetLastError());
   return SCAMP_OK;
 }
@@ -1209,7 +1202,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       CUDA_TRY(cudaEventRecord(ws.evk0, st));
       ws.timed_kernel = true;
     }
-    // ---- bounds pass: joins without seeds start from lower bounds ----
+    // ---- bounds pass: the exact form starts from lower bounds ----
     if (mat_exact) {
       // of every grid entry, in a grid of their own
       void* q;
@@ -1227,10 +1220,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       }
       P.knn_k = static_cast<int>(knn_k);
     }
-    if (exact || (kind == K_MIXED && is_1nn && !seed_a && !use_tc)) {
+    if (kind == K_EXACT) {
       JoinParams B = P;
       B.unit_counter = dcount + 11;
-      if ((rc = launch_bounds(B, exact, grid, smem, st, msg))) return rc;
+      if ((rc = launch_bounds(B, grid, smem, st, msg))) return rc;
       ++launches;
     }
     if (knn_exact) {

@@ -339,9 +339,8 @@ __global__ void join_mixed_knn_kernel(JoinParams P);  // mixed APPROX_ALL_NEIGHB
 __global__ void join_exact_1nn_kernel(JoinParams P);  // FP64 1NN, k-best behind the FP32 filter
 __global__ void join_exact_mat_kernel(JoinParams P);  // FP64 MATRIX_SUMMARY behind it
 __global__ void verify_exact_kernel(JoinParams P);
-// Lower bounds of every window's best before the join itself (FP64 / mixed)
+// Lower bounds of every window's best before the exact form's join
 __global__ void bound_exact_1nn_kernel(JoinParams P);
-__global__ void bound_mixed_1nn_kernel(JoinParams P);
 __global__ void bound_exact_mat_kernel(JoinParams P);  // of every grid entry
 // Per window, the key of the bound of its k-th best: the largest of the
 // threshold, the bounds list's k-th and the given list's k-th.

@@ -43,7 +43,7 @@
 // cell (self-join of 131072 samples, m = 100: 67.5 -> 2.6 ms in the join
 // kernels; 40009 samples with gaps, m = 1024: 39.0 -> 3.4 ms).
 //
-// Bounds pass (bound_*_1nn_kernel), before 1NN joins without seeds: from
+// Bounds pass (bound_exact_1nn_kernel), before double 1NN joins: from
 // nothing, a window's best rises about ln(cells) times and every rise flags
 // its whole 8 x 8 x 2 block, so after k cells per window about 640 / k of the
 // steps are flagged, and a flagged step costs 30 plain ones: below some 10^5
@@ -51,8 +51,10 @@
 // 8000-20000 samples).  The pass walks every 2^14 / ns-th band first, each
 // cell a multiply and a maximum more than the plain filter, and leaves every
 // window a lower bound of its best over 2^14 cells; the join then flags 0.4 -
-// 5% of its steps.  Double, device time: 10007 samples m = 100 0.79 -> 0.29
-// ms, 20000 samples 0.76 -> 0.45 ms.
+// 5% of its steps.  Device time: 10007 samples m = 100 0.79 -> 0.29 ms, 20000
+// samples 0.76 -> 0.45 ms.  Mixed joins go without it: of two cells with equal
+// FP32 values the first one published is the partner, and filters that start
+// high let another one be first (81 of 8937 windows of a noisy sine, m = 64).
 //
 // SUM_THRESH (the reference's sum of every r above the threshold,
 // src/kernels_compute.h:87-113 and 380-392), join_mixed_sum_kernel: every
@@ -133,10 +135,6 @@ constexpr float kAbsSlack = 1.0e-6f;
 // A request whose bound is wider says that FP32 carries nothing there (a
 // large step has passed through the windows); JoinParams::wide_budget.
 constexpr float kWideBound = 1.0f / 8.0f;
-// Mixed form: how far below the FP32 values its bounds pass stays.  Wider
-// than any error of a trusted value, so that a cell near a window's best is
-// still settled by the join itself, as in a join that starts from nothing.
-constexpr float kMixedBoundSlack = 1.0e-3f;
 
 typedef unsigned long long u64;
 
@@ -1025,8 +1023,8 @@ __device__ __forceinline__ void raise_shared(float2& slot, unsigned x, unsigned 
 
 // Raises window w's key to the bound lb > 0 (0: none; then w may lie outside
 // the series).  The key carries no partner: its index field 0 loses every
-// tie, and the cell the bound came from has a larger r (its own FP32 value
-// in the mixed form), so a real cell replaces it.
+// tie, and the cell the bound came from has a larger r, so a real cell
+// replaces it.
 // k-best lists (k > 0): every call's bound comes from cells of its own (a
 // row's in one band, a column's in one unit), so a list of the largest k
 // bounds holds a lower bound of the k-th best.
@@ -1125,7 +1123,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
   static_assert(!(kMat && (kSum || kCoarse)), "the matrix form takes per-cell maxima");
   static_assert(!(kKnn && (kSum || kCoarse || kMat)), "the k-best form is a 1NN variant");
   static_assert(!(kExact && (kSum || kKnn || kCoarse)), "no exact form of these");
-  static_assert(!(kBound && (kSum || kCoarse || kKnn || (kMat && !kExact))), "no bounds of these");
+  static_assert(!kBound || kExact, "bounds are the exact form's");
   constexpr bool kRaise = kBound && !kMat;   // bounds of every window
   constexpr bool kRuns = kMat && (!kExact || kBound);  // running maxima of grid entries
   constexpr bool kWindow = !kRaise && !(kSum && !kCoarse);  // steps carry the column window
@@ -1706,15 +1704,8 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
           float4 cf[kRows + kDiags - 1];
           float2 ci[kRows + kDiags - 1];
           unsigned rmx = 0, rmy = 0;  // lane rr: row rr's bound over the warp (float bits)
-          // exact: the step's bound; mixed: only values the join itself
-          // would take without a direct dot count (margin within kTrust)
-          float2 lo;
-          if constexpr (kExact) {
-            lo = make_float2(fmaf(kBoundSlack, mg.x, kAbsSlack), fmaf(kBoundSlack, mg.y, kAbsSlack));
-          } else {
-            lo = make_float2(kStepMarginC * mg.x <= kTrust ? kMixedBoundSlack : kNoTarget,
-                             kStepMarginC * mg.y <= kTrust ? kMixedBoundSlack : kNoTarget);
-          }
+          const float2 lo = make_float2(fmaf(kBoundSlack, mg.x, kAbsSlack),
+                                        fmaf(kBoundSlack, mg.y, kAbsSlack));
 #pragma unroll
           for (int x = 0; x < kRows + kDiags - 1; ++x) cmax[x] = make_float2(-3.f, -3.f);
 #pragma unroll
@@ -2277,10 +2268,6 @@ __global__ void knn_floor_kernel(const unsigned long long* __restrict__ bounds,
   const uint64_t c = q_from_float_bits(__float_as_uint(__double2float_rd(thr)), kl.frac_bits);
   const uint64_t q = a > b ? (a > c ? a : c) : (b > c ? b : c);
   out[w] = q << kl.idx_bits;
-}
-
-__global__ void __launch_bounds__(kThreads, 4) bound_mixed_1nn_kernel(JoinParams P) {
-  band_body<false, false, false, false, false, true>(P);
 }
 
 // Settles the verification requests of the band kernels, one warp per
