@@ -1917,8 +1917,12 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             const float2 dfr = make_float2(rf.x, rf.y), dgr = make_float2(rf.z, rf.w);
             const float2 ivr = sm.r_iv[r0 + rr];
             // the row's largest cov * inv_c, times inv_r (> 0): the largest r
-            // of the row, rounded exactly as (cov * inv_c) * inv_r per cell
-            float mx = -3.f, my = -3.f;
+            // of the row, rounded exactly as (cov * inv_c) * inv_r per cell.
+            // (From -3 the result is an upper bound only: -3 inv_r where every
+            // r of the row lies below that.  A filter may take it; a grid
+            // entry's maximum and its lower bound have to be a cell's r, and
+            // a row without a cell leaves bx, by at -3.)
+            float mx = kMat ? -INFINITY : -3.f, my = mx;
 #pragma unroll
             for (int k = 0; k < kDiags; k += 2) {
               const float2 pa = mul2(cov[k], ciw[(8 * P + rr + k) & 15]);
@@ -1951,6 +1955,7 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
             const float ub = (g ? by : bx) + fmaf(kBoundSlack, g ? mg.y : mg.x, kAbsSlack);
             if (!(ub > thr)) continue;
             const int64_t i0 = rbase[g] + r0, j0 = i0 + d_my;
+            if (i0 >= pr.R.ns || j0 >= pr.C.ns) continue;  // no cell, no grid entry
             float lo = kNoTarget;
             if (sm.cx.mcol) lo = mat_block_floor(sm.cx, i0, kRows - 1, j0, kRows + kDiags - 2);
             if (sm.cx.mrow)
@@ -1970,9 +1975,10 @@ __device__ __forceinline__ void band_body(const JoinParams& P) {
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
             const float bm = (g ? by : bx) - (g ? sub.y : sub.x);
-            if (!(bm > thr)) continue;
-            tfast = fmaxf(tfast, g ? smg.y : smg.x);
+            if (!((g ? by : bx) > -3.f && bm > thr)) continue;
             const int64_t i0 = rbase[g] + r0, j0 = i0 + d_my;
+            if (i0 >= pr.R.ns || j0 >= pr.C.ns) continue;  // no cell, no grid entry
+            tfast = fmaxf(tfast, g ? smg.y : smg.x);
             const int64_t rpc = sm.cx.rpc, cpc = sm.cx.cpc;
             int cell[2] = {-1, -1};
             bool uni = true;
