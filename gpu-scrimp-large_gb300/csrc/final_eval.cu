@@ -20,8 +20,9 @@
 // terms by FMA into two accumulators of at most ceil(m / 16) terms, one add
 // joins them and three shuffle levels add the lanes' sums, so the dot is off
 // by gamma_{ceil(m/16) + 6} ||x|| ||y||; an inverse norm by 5 u at
-// most (its sum of squares is compensated throughout; then its rounding, a
-// square root and a quotient); two products follow.
+// most (its sum of squares is compensated throughout, and summed directly where
+// the recurrence's residue could show; then its rounding, a square root and a
+// quotient); two products follow.
 // Together at most gamma_{ceil(m/16) + 18}, within the stated
 //   |r_hat - r| <= 2 gamma_{ceil(m/16) + 10}.
 // The 64-bit key then keeps r to 2^-F.  The host adds the two

@@ -198,6 +198,7 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
   sc = __shfl_sync(kAll, sc, 0);
 
   // 32 windows at a time; (ps, pc) and (ss, sc) are those of window wb.
+  int top = 0;  // high word of the chunk's largest sum of squares so far
   for (int64_t wb = w0; wb < w1; wb += 32) {
     const int64_t w = wb + lane;
     const bool active = w < w1;
@@ -260,11 +261,16 @@ __device__ __forceinline__ void stats_body(int64_t chunk, int lane, const double
     const unsigned before = bad & ((1u << lane) - 1u);
     int64_t lb = last_bad;
     if (before) lb = wb + m + (31 - __clz(before));
+    double ssd = ssd_s + ssd_c;
+    top = max(top, static_cast<int>(__reduce_max_sync(
+                       kAll, active ? static_cast<unsigned>(max(__double2hiint(ssd), 0)) : 0u)));
     if (active) {
-      // A near-flat ssd from the recurrence is summed again directly, so the
-      // flatness rule sees no accumulated residue.
-      double ssd = ssd_s + ssd_c;
-      if (ssd <= 1e3 * kFlatnessEpsilon) {
+      // Summed again directly, so that no accumulated residue shows: a
+      // near-flat ssd (for the flatness rule), and one 2^40 below the largest
+      // of its chunk, of which the recurrence keeps 2^-104 (unit noise, m =
+      // 100, behind a spike of 1e10 349 u of the ssd, of 1e14 2.5e-6; now 2^-64
+      // of it at most).
+      if (ssd <= 1e3 * kFlatnessEpsilon || (top >> 20) - (__double2hiint(ssd) >> 20) > 40) {
         double s2 = 0, c2 = 0;
         for (int64_t t = 0; t < m; ++t) {
           const double v = (clean(T_raw[w + t]) - mu) - mu_lo;
