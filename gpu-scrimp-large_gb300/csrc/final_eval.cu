@@ -22,7 +22,9 @@
 // by gamma_{ceil(m/16) + 6} ||x|| ||y||; an inverse norm by 5 u at
 // most (its sum of squares is compensated throughout, and summed directly where
 // the recurrence's residue could show; then its rounding, a square root and a
-// quotient); two products follow.
+// quotient); two products follow.  (The means' own rounding adds m times the
+// product of two of them, second order: it shows where a series' offset is 10^8
+// and more times its windows' deviation.)
 // Together at most gamma_{ceil(m/16) + 18}, within the stated
 //   |r_hat - r| <= 2 gamma_{ceil(m/16) + 10}.
 // The 64-bit key then keeps r to 2^-F.  The host adds the two

@@ -1,10 +1,11 @@
-"""GPU: norms behind very large samples, and the correlations reported with
-them.
+"""GPU: norms behind very large samples and on large offsets, and the
+correlations reported with them.
 
 The statistics' sums of squares run on from window to window for 64 windows: a
 spike of S standard deviations must leave nothing of its S^2 in the windows
-behind it.  Exact values in rational arithmetic; the reported correlation is held
-to the error bound that the call states (and 1e-15 for the check's own rounding).
+behind it, and the rounding of an offset's mean nothing in any.  Exact values in
+rational arithmetic; the reported correlation is held to the error bound that
+the call states (and 1e-15 for the check's own rounding).
 """
 import math
 from fractions import Fraction
@@ -28,6 +29,11 @@ def spiked(n, size, seed):
 @pytest.mark.parametrize("size", [1e8, 1e10, 1e12, 1e14, 1e18])
 def test_norms_behind_spikes(gpu_engine, size, m):
     check(gpu_engine, spiked(2100, size, 5), m)
+
+
+@pytest.mark.parametrize("offset,spread", [(1e9, 1.0), (1e9, 1e-2), (-1e12, 1.0)])
+def test_norms_on_offsets(gpu_engine, offset, spread):
+    check(gpu_engine, offset + spread * np.random.default_rng(6).standard_normal(2100), 100)
 
 
 @pytest.mark.parametrize("precision", ["double", "mixed"])
