@@ -406,6 +406,8 @@ struct Workspace {
   // join; requests beyond the capacity are verified inline, more slowly).
   int64_t vreq_cap = 0;
   int64_t vreq_seen = 0;
+  int64_t vreq_worth = INT64_MAX;  // most that the last join would have used
+  bool exact = false;              // whether the last join ran the exact form
   // Batched joins: the executable graph of the last batch layout (replayed
   // while the layout repeats) and the autotuned segment length per window.
   cudaGraphExec_t batch_exec = nullptr;
@@ -418,6 +420,11 @@ struct Workspace {
 
 constexpr int64_t kMinVerifyReqs = int64_t{1} << 22;
 constexpr int64_t kMaxVerifyReqs = int64_t{1} << 30;  // 16 GiB of requests
+// Smallest request buffer on a device that has no room for more.
+constexpr int64_t kLeastVerifyReqs = int64_t{1} << 12;
+// Largest one that a join of the exact form leaves in the workspace (1 GiB;
+// joins that ask for more take 100 ms and more, their allocation 1 ms).
+constexpr int64_t kKeptVerifyReqs = int64_t{1} << 26;
 
 Workspace g_ws[64];
 
@@ -471,6 +478,36 @@ enum Slot {
   S_TC_TAB, S_TC_W, S_TC_XS, S_TC_RAW, S_TC_OUT, S_TC_XI, S_FP64_LIST,
   S_FP64_UNIT, S_KNN_BOUND_A, S_KNN_BOUND_B, S_MAT_BOUND,
 };
+
+// Gives a buffer back (cudaFree waits for the work that uses it).
+void release(Workspace& ws, size_t slot) {
+  if (slot >= ws.bufs.size() || !ws.bufs[slot].p) return;
+  cudaFree(ws.bufs[slot].p);
+  ws.bufs[slot] = Buf{};
+}
+
+// The request buffer: `want` requests, or the largest half, quarter, ... of
+// them that the device has room for: requests past its end are verified in
+// place (mixed forms), their units left to the FP64 kernels (exact form).
+int ensure_requests(Workspace& ws, int64_t want, VerifyReq** out, std::string* msg) {
+  int rc;
+  void* p;
+  while ((rc = ensure(ws, S_VREQ, static_cast<size_t>(want) * sizeof(VerifyReq), &p, msg))) {
+    ws.vreq_cap = 0;
+    if (rc != SCAMP_ERR_OUT_OF_MEMORY || want <= kLeastVerifyReqs) return rc;
+    want /= 2;
+  }
+  ws.vreq_cap = want;
+  *out = static_cast<VerifyReq*>(p);
+  return SCAMP_OK;
+}
+
+// The exact form's own buffers beside what the FP64 kernels need.
+void release_exact(Workspace& ws) {
+  for (size_t slot : {S_VREQ, S_FP64_LIST, S_FP64_UNIT, S_KNN_BOUND_A, S_KNN_BOUND_B, S_MAT_BOUND})
+    release(ws, slot);
+  ws.vreq_cap = 0;
+}
 
 #define CUDA_TRY(expr)                                                     \
   do {                                                                     \
@@ -725,7 +762,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                const double* dA, const double* dB, uint64_t* dprof_a,
                uint64_t* dprof_b, double* dsum_a, double* dsum_b,
                double* dcorr_a, double* dcorr_b, cudaStream_t st,
-               std::string* msg, bool nested = false, const ExtraOut* ex = nullptr);
+               std::string* msg, bool nested = false, const ExtraOut* ex = nullptr,
+               bool exact_allowed = true);
 
 // Block-averaged join of the inputs (window m / 8) into the seed profiles
 // S_SEED_A/B; returns their device pointers (seed_b null when not kept).
@@ -786,7 +824,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                const double* dA, const double* dB, uint64_t* dprof_a,
                uint64_t* dprof_b, double* dsum_a, double* dsum_b,
                double* dcorr_a, double* dcorr_b, cudaStream_t st,
-               std::string* msg, bool nested, const ExtraOut* ex) {
+               std::string* msg, bool nested, const ExtraOut* ex, bool exact_allowed) {
   scamp_c_args a_local;
   if (a->profile_type == SCAMP_PROFILE_MATRIX_SUMMARY) {
     // matrix summaries reduce along the columns only (src/common.cpp:98-105)
@@ -824,7 +862,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   // 50 x 50 entries: 6.9 and 0.7 ms; 2000 samples, m = 32: five best 1.25 and
   // 0.53 ms, one 0.23 and 0.22.
   const bool fp64_exact = a->precision_type == SCAMP_PRECISION_DOUBLE && !nested &&
-                          plan.m <= kExactMaxWindow;
+                          exact_allowed && plan.m <= kExactMaxWindow;
   const bool mat_exact = is_mat && fp64_exact && mat_rpc >= kMatMixedMinSpan &&
                          mat_cpc >= kMatMixedMinSpan &&
                          std::max(plan.ns_a, plan.ns_b) < (int64_t{1} << 31) &&
@@ -1190,12 +1228,9 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
         want = std::min<int64_t>(want, std::min<int64_t>(kMaxListReqs, std::max(kMinVerifyReqs, worth)));
       want = std::max<int64_t>(want, ws.vreq_seen + ws.vreq_seen / 4);
       want = std::max<int64_t>(std::min<int64_t>(want, kMaxVerifyReqs), ws.vreq_cap);
-      void* q;
-      if ((rc = ensure(ws, S_VREQ, static_cast<size_t>(want) * sizeof(VerifyReq), &q, msg)))
-        return rc;
-      ws.vreq_cap = want;
-      P.vreq = static_cast<VerifyReq*>(q);
-      P.vreq_cap = std::min<int64_t>(want, worth);
+      if ((rc = ensure_requests(ws, want, &P.vreq, msg))) return rc;
+      P.vreq_cap = std::min<int64_t>(ws.vreq_cap, worth);
+      ws.vreq_worth = worth;
     }
     const int64_t grid = std::min<int64_t>(resident, P.total_units);
     if (!nested) {
@@ -1472,10 +1507,29 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
     res->max_tie_margin = (fp64_final && kind == K_MIXED) ? 0.0 : -1.0;
   }
   if (!nested) {
+    ws.exact = kind == K_EXACT;
     ws.tracked_sum_margin = !is_1nn && !knn_mixed && kind == K_MIXED;
     ws.tracked_tie_margin = (is_1nn || knn_mixed) && kind == K_MIXED;
   }
   return SCAMP_OK;
+}
+
+// run_device() for the two entries.  The exact form is faster than the FP64
+// and visit kernels but not necessary: where the device has no room for its
+// buffers (nothing of the results is written before all of them are there),
+// they are given back and the join runs without it.
+int run_join(Workspace& ws, const scamp_c_args* a, scamp_c_result* res, const double* dA,
+             const double* dB, uint64_t* const (&prof)[2], double* const (&sum)[2],
+             double* const (&corr)[2], cudaStream_t st, std::string* msg, const ExtraOut* ex) {
+  for (bool exact_allowed : {true, false}) {
+    const int rc = run_device(ws, a, res, dA, dB, prof[0], prof[1], sum[0], sum[1], corr[0], corr[1],
+                              st, msg, false, ex, exact_allowed);
+    if (rc != SCAMP_ERR_OUT_OF_MEMORY || !exact_allowed ||
+        a->precision_type != SCAMP_PRECISION_DOUBLE)
+      return rc;
+    release_exact(ws);
+  }
+  return SCAMP_OK;  // not reached
 }
 
 // Timing fields, work counters and the device error word of the last join
@@ -1491,7 +1545,8 @@ int read_times(Workspace& ws, scamp_c_result* res, std::string* msg = nullptr) {
       res->slow_steps = c[2];
       res->verifications = c[3];
       res->inplace_verifications = static_cast<uint32_t>(std::min<unsigned long long>(c[7], UINT32_MAX));
-      ws.vreq_seen = std::max<int64_t>(ws.vreq_seen, static_cast<int64_t>(c[4] + c[7]));
+      ws.vreq_seen = std::max<int64_t>(
+          ws.vreq_seen, std::min<int64_t>(ws.vreq_worth, static_cast<int64_t>(c[4] + c[7])));
       float tm;
       const uint32_t bits = static_cast<uint32_t>(c[5]);
       std::memcpy(&tm, &bits, 4);
@@ -1502,6 +1557,10 @@ int read_times(Workspace& ws, scamp_c_result* res, std::string* msg = nullptr) {
         if (msg) *msg = "Error: a wait on the tensor cores timed out on the device";
       }
     }
+  }
+  if (ws.exact && ws.vreq_cap > kKeptVerifyReqs) {  // (the join has ended)
+    release(ws, S_VREQ);
+    ws.vreq_cap = 0;
   }
   float ms = 0;
   cudaEventElapsedTime(&ms, ws.ev0, ws.ev1);
@@ -1678,9 +1737,9 @@ extern "C" int scamp_gb300_join_dev(const scamp_c_args* args, scamp_c_result* re
   ex.knn[0] = res->knn_a;
   ex.knn[1] = res->knn_b;
   ex.matrix = res->matrix;
-  rc = run_device(*ws, args, res, args->timeseries_a, args->has_b ? args->timeseries_b : args->timeseries_a,
-                  res->profile_a, res->profile_b, res->sum_a, res->sum_b, res->corr_a, res->corr_b, st, &msg,
-                  false, &ex);
+  rc = run_join(*ws, args, res, args->timeseries_a, args->has_b ? args->timeseries_b : args->timeseries_a,
+                {res->profile_a, res->profile_b}, {res->sum_a, res->sum_b}, {res->corr_a, res->corr_b}, st,
+                &msg, &ex);
   if (rc == SCAMP_OK) {
     cudaError_t e = cudaEventSynchronize(ws->ev1);
     if (e != cudaSuccess) { msg = std::string("CUDA error: ") + cudaGetErrorString(e); rc = SCAMP_ERR_CUDA; }
@@ -1779,10 +1838,9 @@ extern "C" int scamp_gb300_join(const scamp_c_args* args, scamp_c_result* res,
       HOST_CUDA(cudaMemcpyAsync(p, hsum[s], nsz[s] * 8, cudaMemcpyHostToDevice, st));
     }
   }
-  rc = run_device(*ws, args, res, static_cast<double*>(pa),
-                  args->has_b ? static_cast<double*>(pb) : static_cast<double*>(pa),
-                  dprof[0], dprof[1], dsum[0], dsum[1], dcorr[0], dcorr[1], st, &msg,
-                  false, &ex);
+  rc = run_join(*ws, args, res, static_cast<double*>(pa),
+                args->has_b ? static_cast<double*>(pb) : static_cast<double*>(pa), dprof, dsum, dcorr, st,
+                &msg, &ex);
   if (rc) return fail(rc);
   if (matrix) HOST_CUDA(cudaMemcpyAsync(res->matrix, ex.matrix, mat_n * 4, cudaMemcpyDeviceToHost, st));
   for (int s = 0; s < 2 && !matrix; ++s) {
@@ -2488,6 +2546,7 @@ int run_batch(Workspace& ws, const scamp_c_args* args, scamp_c_result* res, int 
       std::min<int64_t>((wpre.back() + 31) / 32, static_cast<int64_t>(ws.sms) * 16), 1);
   const int64_t seed_blocks = std::max<int64_t>(
       std::min<int64_t>((wpre.back() + 255) / 256, static_cast<int64_t>(ws.sms) * 32), 1);
+  ws.exact = false;
   JoinParams P{};
   int64_t grid = 0;
   const size_t smem = mixed_1nn_smem_bytes();
@@ -2508,11 +2567,8 @@ int run_batch(Workspace& ws, const scamp_c_args* args, scamp_c_result* res, int 
     int64_t want = std::max<int64_t>(kMinVerifyReqs, 32 * Nns);
     want = std::max<int64_t>(want, ws.vreq_seen + ws.vreq_seen / 4);
     want = std::max<int64_t>(std::min<int64_t>(want, kMaxVerifyReqs), ws.vreq_cap);
-    void* q;
-    if ((rc = ensure(ws, S_VREQ, static_cast<size_t>(want) * sizeof(VerifyReq), &q, msg))) return rc;
-    ws.vreq_cap = want;
-    P.vreq = static_cast<VerifyReq*>(q);
-    P.vreq_cap = want;
+    if ((rc = ensure_requests(ws, want, &P.vreq, msg))) return rc;
+    P.vreq_cap = ws.vreq_cap;
     CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     int occ = 1;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, mixed_1nn_threads(), smem));
