@@ -53,8 +53,8 @@ __device__ __forceinline__ int64_t ord_double(double x) {
 }
 
 // SUM_THRESH adds in fixed point: r as a signed integer in units of 2^-53
-// (the last place of r in [1/2, 1), the bits below cut off), integer pipe
-// only.  Integer sums are exact, so a slab's sum (at most 512 cells, |r| <= 1
+// (the last place of r in [1/2, 1); smaller ones rounded to it, not cut, which
+// would take 2^-55 and more from every term), integer pipe only.  Integer sums are exact, so a slab's sum (at most 512 cells, |r| <= 1
 // up to rounding: 2^62) carries less error than one added in FP64, and they
 // leave the FP64 pipe the recurrence's four operations per cell: the two
 // additions per cell and the row reductions' shuffles in FP64 had taken three
@@ -69,7 +69,7 @@ __device__ __forceinline__ long long fixed_r(double r) {
   const uint64_t sig = (bits & 0x000FFFFFFFFFFFFFull) | (e ? (1ull << 52) : 0);
   const int s = 1075 - kSumFrac - e;  // |r| 2^53 = sig 2^-s
   constexpr uint64_t kMost = 3ull << (kSumFrac - 1);
-  uint64_t mag = s >= 64 ? 0 : (s >= 0 ? sig >> s : (s == -1 ? sig << 1 : kMost));
+  uint64_t mag = s >= 64 ? 0 : (s >= 0 ? (((sig << 1) >> s) + 1) >> 1 : (s == -1 ? sig << 1 : kMost));
   if (mag > kMost) mag = kMost;
   return (bits >> 63) ? -static_cast<long long>(mag) : static_cast<long long>(mag);
 }
