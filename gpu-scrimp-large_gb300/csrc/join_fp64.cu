@@ -95,80 +95,71 @@ struct SmemFp64 {
   long long unit;
 };
 
-// Covariance of row window i and column window j, each centred by its own
-// mean (the reference's QT seed, src/qt_helper.cpp:52-72).
-__device__ __noinline__ double seed_own(const SeriesDev& R, const SeriesDev& C, int64_t i,
-                                        int64_t j, int64_t m) {
-  const double mr = R.mean[i], mc = C.mean[j];
-  const double* __restrict__ tr = R.T + i;
-  const double* __restrict__ tc = C.T + j;
-  double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-  int64_t t = 0;
-  for (; t + 4 <= m; t += 4) {
-    a0 = fma(tr[t] - mr, tc[t] - mc, a0);
-    a1 = fma(tr[t + 1] - mr, tc[t + 1] - mc, a1);
-    a2 = fma(tr[t + 2] - mr, tc[t + 2] - mc, a2);
-    a3 = fma(tr[t + 3] - mr, tc[t + 3] - mc, a3);
-  }
-  for (; t < m; ++t) a0 = fma(tr[t] - mr, tc[t] - mc, a0);
-  return (a0 + a1) + (a2 + a3);
-}
-
 // FP64 direct-dot seeds: the covariances of row window i with the column
-// windows j .. j + kDiags - 1.  The row window is centred by its own mean, the
+// windows j .. j + kDiags - 1 (the reference's QT seed,
+// src/qt_helper.cpp:52-72).  The row window is centred by its own mean, the
 // column samples by the first window's, which the four windows share:
 //   cov_k = sum x_t y_{t+k} - (mean_{j+k} - mean_j) sum x_t,
-// 7 FP64 operations per sample for four windows against 12 with each window
+// 7 FP64 operations per sample for four windows against 9 with each window
 // centred by itself.  The products then carry the means' difference, so each
-// window is centred by itself (seed_own) where that exceeds 1/4 of a window's
-// standard deviation, beside which it adds 3% to the rounding (a spike, or a
-// gap on an offset, that leaves with the first window), and where a window
-// has no inverse norm to tell.  (At 1/8 random walks cross it: 32768 samples,
-// m = 128, 5.18 ms against 5.09, which it also takes without the test.)
-// Windows at or past C.ns get 0.
+// window is centred by itself where that exceeds 1/4 of a window's standard
+// deviation in some lane of the warp (beside 1/4 it adds 3% to the rounding; a
+// spike, or a gap on an offset, that leaves with the first window carries any
+// amount), and where a window has no inverse norm to tell.  At 1/8 random
+// walks cross it: 32768 samples, m = 128, 5.18 ms against 5.09, which it also
+// takes without the test.  Windows at or past C.ns get 0.  Called by whole
+// warps.
 __device__ __forceinline__ void seed_fp64(const SeriesDev& R, const SeriesDev& C, int64_t i,
                                           int64_t j, int64_t m, double (&cov)[kDiags]) {
-#pragma unroll
-  for (int k = 0; k < kDiags; ++k) cov[k] = 0.0;
-  if (j >= C.ns) return;
-  const double mr = R.mean[i], mc = C.mean[j];
+  const double mr = R.mean[i];
+  double mc[kDiags];
   bool near = true;
 #pragma unroll
-  for (int k = 1; k < kDiags; ++k) {
-    if (j + k >= C.ns) break;
-    const double shift = (C.mean[j + k] - mc) * C.inv[j + k];
-    near = near && shift * shift * static_cast<double>(m) <= 1.0 / 16.0;
-  }
-  if (!near) {
-#pragma unroll 1
-    for (int k = 0; k < kDiags; ++k) {
-      const double v = j + k < C.ns ? seed_own(R, C, i, j + k, m) : 0.0;
-#pragma unroll
-      for (int q = 0; q < kDiags; ++q)
-        if (q == k) cov[q] = v;
+  for (int k = 0; k < kDiags; ++k) {
+    cov[k] = 0.0;
+    mc[k] = j + k < C.ns ? C.mean[j + k] : 0.0;
+    if (k > 0 && j + k < C.ns) {
+      const double shift = (mc[k] - mc[0]) * C.inv[j + k];
+      near = near && shift * shift * static_cast<double>(m) <= 1.0 / 16.0;
     }
-    return;
   }
+  near = __all_sync(0xffffffffu, near);
+  if (j >= C.ns) return;
   const double* __restrict__ tr = R.T + i;
   const double* __restrict__ tc = C.T + j;
   const int64_t nc = C.n - j;  // column samples from j on
+  const double shared = near ? mc[0] : 0.0;
   double xs = 0.0;
   double y[kDiags];
 #pragma unroll
-  for (int k = 0; k + 1 < kDiags; ++k) y[k] = k < nc ? tc[k] - mc : 0.0;
+  for (int k = 0; k + 1 < kDiags; ++k) y[k] = k < nc ? tc[k] - shared : 0.0;
+  if (near) {
 #pragma unroll 4
-  for (int64_t t = 0; t < m; ++t) {
-    const double x = tr[t] - mr;
-    y[kDiags - 1] = t + kDiags - 1 < nc ? tc[t + kDiags - 1] - mc : 0.0;
-    xs += x;
+    for (int64_t t = 0; t < m; ++t) {
+      const double x = tr[t] - mr;
+      y[kDiags - 1] = t + kDiags - 1 < nc ? tc[t + kDiags - 1] - shared : 0.0;
+      xs += x;
 #pragma unroll
-    for (int k = 0; k < kDiags; ++k) cov[k] = fma(x, y[k], cov[k]);
+      for (int k = 0; k < kDiags; ++k) cov[k] = fma(x, y[k], cov[k]);
 #pragma unroll
-    for (int k = 0; k + 1 < kDiags; ++k) y[k] = y[k + 1];
+      for (int k = 0; k + 1 < kDiags; ++k) y[k] = y[k + 1];
+    }
+#pragma unroll
+    for (int k = 0; k < kDiags; ++k) cov[k] = fma(-(mc[k] - shared), xs, cov[k]);
+  } else {
+#pragma unroll 4
+    for (int64_t t = 0; t < m; ++t) {
+      const double x = tr[t] - mr;
+      y[kDiags - 1] = t + kDiags - 1 < nc ? tc[t + kDiags - 1] : 0.0;
+#pragma unroll
+      for (int k = 0; k < kDiags; ++k) cov[k] = fma(x, y[k] - mc[k], cov[k]);
+#pragma unroll
+      for (int k = 0; k + 1 < kDiags; ++k) y[k] = y[k + 1];
+    }
   }
 #pragma unroll
   for (int k = 0; k < kDiags; ++k)
-    cov[k] = j + k < C.ns ? fma(-(C.mean[j + k] - mc), xs, cov[k]) : 0.0;
+    if (j + k >= C.ns) cov[k] = 0.0;
 }
 
 }  // namespace
