@@ -170,6 +170,19 @@ constexpr int64_t kWidePerCells = 1024;
 // samples of a sine, m = 1024, 3.2 requests per cell over m: 7.7 ms, with a limit
 // of 2 10.1, of 1 12.9); random walks make 1.0 and fewer.
 constexpr double kExactReqs = 4.0;
+// The same of a matrix summary, whose ordinary series make 0.5 and fewer (60000
+// samples of a square wave, m = 500, 100 x 100 entries: 105 ms without a limit,
+// 34 with it, visit kernel alone 28.6).
+constexpr double kMatReqs = 1.0;
+// Their buffer, in requests per window of both series.  It has to hold what
+// ordinary series ask for, which rises with the join's length (walks, m = 1024:
+// 86 per window of a self-join at 2^19 samples, 102 at 2^20; with gaps 100 at
+// 2^19), or units are left to FP64: 64 are enough below 2^18 windows, above them
+// walks with noise of 2^20 samples take 1470 ms with 64 and 176 with 128. More
+// is lost where no bound separates the cells: square wave, 60000 samples, m =
+// 256, 18 ms with 64 and 33 with 128, FP64 band kernel alone 22; 2^19 samples, m
+// = 1024, 1078 and 1090 ms.
+int64_t exact_reqs(int64_t windows) { return windows * (windows < (int64_t{1} << 19) ? 64 : 128); }
 
 // Requests of a k-best join in all, per cell over the window length; the units
 // beyond them are left to the visit kernel, whose time grows with k.  No
@@ -406,8 +419,8 @@ struct Workspace {
   // join; requests beyond the capacity are verified inline, more slowly).
   int64_t vreq_cap = 0;
   int64_t vreq_seen = 0;
-  int64_t vreq_worth = INT64_MAX;  // most that the last join would have used
-  bool exact = false;              // whether the last join ran the exact form
+  bool exact = false;       // whether the last join ran the exact form
+  bool vreq_grown = false;  // and enlarged the buffer
   // Batched joins: the executable graph of the last batch layout (replayed
   // while the layout repeats) and the autotuned segment length per window.
   cudaGraphExec_t batch_exec = nullptr;
@@ -422,7 +435,7 @@ constexpr int64_t kMinVerifyReqs = int64_t{1} << 22;
 constexpr int64_t kMaxVerifyReqs = int64_t{1} << 30;  // 16 GiB of requests
 // Smallest request buffer on a device that has no room for more.
 constexpr int64_t kLeastVerifyReqs = int64_t{1} << 12;
-// Largest one that a join of the exact form leaves in the workspace (1 GiB;
+// Largest one that a join of the exact form enlarges it to for good (1 GiB;
 // joins that ask for more take 100 ms and more, their allocation 1 ms).
 constexpr int64_t kKeptVerifyReqs = int64_t{1} << 26;
 
@@ -878,6 +891,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
 
   if (!nested) {
     ws.timed_kernel = false;
+    ws.vreq_grown = false;
     ws.timed_verify = false;
     // the tensor-core anchors' one-time self-check (before this join's own
     // statistics, whose buffers it borrows)
@@ -1218,19 +1232,24 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       // ask for more)
       int64_t want = std::max<int64_t>(kMinVerifyReqs, 32 * (nsz[0] + nsz[1]) *
                                                            (knn_mixed || knn_exact ? 4 * knn_k : 1));
-      const double per_cell = knn_exact ? list_reqs(knn_k)
-                            : kind == K_EXACT && is_1nn ? kExactReqs : 0.0;
-      const int64_t worth = per_cell > 0.0
-          ? static_cast<int64_t>(per_cell * cells_d / static_cast<double>(m)) +
-                (knn_exact ? kListReqsLatency / m : 256 * resident)
-          : INT64_MAX;
-      if (knn_exact)
-        want = std::min<int64_t>(want, std::min<int64_t>(kMaxListReqs, std::max(kMinVerifyReqs, worth)));
-      want = std::max<int64_t>(want, ws.vreq_seen + ws.vreq_seen / 4);
+      // Exact form: no more than are worth verifying, whatever the buffer an
+      // earlier join has left.
+      int64_t most = INT64_MAX;
+      if (kind == K_EXACT) {
+        const double per_cell = knn_exact ? list_reqs(knn_k) : is_1nn ? kExactReqs : kMatReqs;
+        const int64_t worth = static_cast<int64_t>(per_cell * cells_d / static_cast<double>(m)) +
+                              (knn_exact ? kListReqsLatency / m : 256 * resident);
+        if (knn_exact) want = std::min<int64_t>(want, kMaxListReqs);
+        if (is_1nn) want = std::max<int64_t>(want, exact_reqs(nsz[0] + nsz[1]));
+        most = std::min(want, worth);
+        want = std::min<int64_t>(want, std::max(kMinVerifyReqs, worth));
+      } else {
+        want = std::max<int64_t>(want, ws.vreq_seen + ws.vreq_seen / 4);
+      }
       want = std::max<int64_t>(std::min<int64_t>(want, kMaxVerifyReqs), ws.vreq_cap);
+      ws.vreq_grown = kind == K_EXACT && want > ws.vreq_cap;
       if ((rc = ensure_requests(ws, want, &P.vreq, msg))) return rc;
-      P.vreq_cap = std::min<int64_t>(ws.vreq_cap, worth);
-      ws.vreq_worth = worth;
+      P.vreq_cap = std::min(ws.vreq_cap, most);
     }
     const int64_t grid = std::min<int64_t>(resident, P.total_units);
     if (!nested) {
@@ -1545,8 +1564,8 @@ int read_times(Workspace& ws, scamp_c_result* res, std::string* msg = nullptr) {
       res->slow_steps = c[2];
       res->verifications = c[3];
       res->inplace_verifications = static_cast<uint32_t>(std::min<unsigned long long>(c[7], UINT32_MAX));
-      ws.vreq_seen = std::max<int64_t>(
-          ws.vreq_seen, std::min<int64_t>(ws.vreq_worth, static_cast<int64_t>(c[4] + c[7])));
+      if (!ws.exact)
+        ws.vreq_seen = std::max<int64_t>(ws.vreq_seen, static_cast<int64_t>(c[4] + c[7]));
       float tm;
       const uint32_t bits = static_cast<uint32_t>(c[5]);
       std::memcpy(&tm, &bits, 4);
@@ -1558,7 +1577,7 @@ int read_times(Workspace& ws, scamp_c_result* res, std::string* msg = nullptr) {
       }
     }
   }
-  if (ws.exact && ws.vreq_cap > kKeptVerifyReqs) {  // (the join has ended)
+  if (ws.vreq_grown && ws.vreq_cap > kKeptVerifyReqs) {  // (the join has ended)
     release(ws, S_VREQ);
     ws.vreq_cap = 0;
   }
@@ -2546,7 +2565,7 @@ int run_batch(Workspace& ws, const scamp_c_args* args, scamp_c_result* res, int 
       std::min<int64_t>((wpre.back() + 31) / 32, static_cast<int64_t>(ws.sms) * 16), 1);
   const int64_t seed_blocks = std::max<int64_t>(
       std::min<int64_t>((wpre.back() + 255) / 256, static_cast<int64_t>(ws.sms) * 32), 1);
-  ws.exact = false;
+  ws.exact = ws.vreq_grown = false;
   JoinParams P{};
   int64_t grid = 0;
   const size_t smem = mixed_1nn_smem_bytes();

@@ -11,6 +11,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -56,3 +57,18 @@ def test_little_memory(gpu_engine, kind, n, m, k, mib):
                         kind, str(n), str(m), str(k), str(mib)],
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "same", r.stdout + r.stderr
+
+
+def test_requests_do_not_depend_on_earlier_joins(gpu_engine):
+    """A join verifies what is worth it at its size, whatever buffer an earlier
+    join has left: a square wave (no bound separates its cells) asks for all it
+    may."""
+    a = (np.arange(60000) // 25 % 2).astype(float)
+
+    def verified():
+        return gpu_engine.join(a, None, 256, precision="double")["counters"]["verifications"]
+
+    before = verified()
+    gpu_engine.join(np.cumsum(np.random.default_rng(1).standard_normal(1 << 18)), None, 64,
+                    precision="double")
+    assert 0 < before and verified() <= 1.2 * before
