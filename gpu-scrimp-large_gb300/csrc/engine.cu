@@ -201,6 +201,17 @@ int64_t exact_reqs(int64_t windows) { return windows * (windows < (int64_t{1} <<
 constexpr int64_t kListReqsLatency = int64_t{1} << 29;
 double list_reqs(int64_t k) { return 3.0 + 0.75 * static_cast<double>(k); }
 constexpr int64_t kMaxListReqs = int64_t{1} << 27;  // 2 GiB of requests
+// Whether the exact form serves lists of k.  Long lists of long windows ask for
+// more than the limit: neighbouring windows match the same places, and where
+// the k best take up much of the series no bound separates them from the rest.
+// 30000-sample walks / beats (visit kernel, exact form): m = 256, 32 best 36.6 and
+// 32.1 / 38.6 and 10.8 ms, 48 best 52.4 and 56.1 / 61.5 and 92.3; m = 500, 20 best
+// 32.6 and 25.9 / 29.2 and 9.7, 32 best 41.2 and 43.3 / 43.1 and 73.7; m = 1000, 16
+// best 42.4 and 33.6 / 38.5 and 31.1, 32 best 51.1 and 56.0 / 50.6 and 82.0; 100000
+// samples, m = 1000, 32 best 272 and 152 / 247 and 73.
+bool exact_list(int64_t k, int64_t m, int64_t windows) {
+  return k <= 16 || k * m <= 8192 || 3 * k * m <= windows;
+}
 
 // Rows between seeds of the FP64 form.  The FP64 recurrence drifts by
 // ~2^-53 per row, so seeds only bound the work lost to them: 32 m rows keep
@@ -880,7 +891,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
                          mat_cpc >= kMatMixedMinSpan &&
                          std::max(plan.ns_a, plan.ns_b) < (int64_t{1} << 31) &&
                          static_cast<int64_t>(a->matrix_height) * a->matrix_width < (int64_t{1} << 31);
-  const bool knn_exact = is_knn && fp64_exact && a->max_matches_per_column <= knn_mixed_max_k();
+  const bool knn_exact = is_knn && fp64_exact && a->max_matches_per_column <= knn_mixed_max_k() &&
+                         exact_list(a->max_matches_per_column, plan.m, std::max(plan.ns_a, plan.ns_b));
   const bool visit = (is_knn && !knn_mixed && !knn_exact) || (is_mat && !mat_mixed && !mat_exact);
   const bool ultra = a->precision_type == SCAMP_PRECISION_ULTRA;
   const int64_t m = plan.m;

@@ -52,3 +52,16 @@ def test_grids(gpu_engine, precision, tol, nb, thr):
     got = gpu_engine.join(a, b, 100, "MATRIX_SUMMARY", precision, **kw)
     assert got["counters"]["steps"] > 0 and want["counters"]["steps"] == 0
     agree(got["matrix"].astype(np.float64), want["matrix"].astype(np.float64), thr, tol)
+
+
+@pytest.mark.parametrize("k", [16, 17])
+def test_either_side_of_the_list_line(gpu_engine, k):
+    """Lists of more than 16 from long windows of a short series go to the visit
+    kernel itself; the values are the same on both sides of the line."""
+    a, m, thr = series(12000, 5), 600, 0.4
+    kw = dict(threshold=thr, max_matches=k)
+    want = gpu_engine.join(a, None, m, "ALL_NEIGHBORS", "ultra", **kw)
+    got = gpu_engine.join(a, None, m, "ALL_NEIGHBORS", "double", **kw)
+    assert (got["counters"]["steps"] > 0) == (k == 16)
+    cw, cg = (gpu_engine.unpack_profile(r["knn_a"])[0].astype(np.float64) for r in (want, got))
+    agree(cg, cw, thr, TOL)
