@@ -324,12 +324,13 @@ def _batch_args(series, windows, precision, device):
         ca = _args(arrs[0], None, windows[0], "1NN_INDEX", precision, True, True, False, False,
                    0.0, -1, -1, 128000, 0, device, True)
         ms = [int(m) for m in windows]
+        u64 = (1 << 64) - 1  # as ctypes stores them: the engine refuses what is no window
         rows = np.frombuffer(cargs, dtype=_lib.CArgs)
         rows[:] = np.frombuffer(ca, dtype=_lib.CArgs)[0]
         rows["timeseries_a"] = [x.ctypes.data for x in arrs]
         rows["len_a"] = [len(x) for x in arrs]
-        rows["window"] = ms
-        rows["max_tile_size"] = [max(128000, 2 * m) for m in ms]
+        rows["window"] = [m & u64 for m in ms]
+        rows["max_tile_size"] = [max(128000, 2 * m) & u64 for m in ms]
     return arrs, windows, cargs
 
 
