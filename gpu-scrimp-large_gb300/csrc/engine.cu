@@ -859,7 +859,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   }
   Plan plan = make_plan(a);
   // 1NN (float best correlation, no index) runs as 1NN_INDEX on the keys;
-  // the k-best and matrix-summary types run the FP64 visit kernel
+  // the k-best and matrix-summary types run the band kernel (mixed and
+  // exact form) or the FP64 visit kernels, see below
   const bool max_only = a->profile_type == SCAMP_PROFILE_1NN;
   const bool is_1nn = a->profile_type == SCAMP_PROFILE_1NN_INDEX || max_only;
   const bool mixed = a->precision_type == SCAMP_PRECISION_MIXED ||
@@ -867,7 +868,8 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   // MATRIX_SUMMARY grid: rows are windows of B (of A in a self-join),
   // columns windows of A.  The mixed form takes the band kernel's per-cell
   // maxima when grid entries span enough windows that most of its 8 x 15
-  // blocks fall inside one; else (and in FP64) the visit kernel serves it.
+  // blocks fall inside one, and so does the exact form; else (and in ULTRA)
+  // the visit kernel serves it.
   const bool is_mat = a->profile_type == SCAMP_PROFILE_MATRIX_SUMMARY;
   const int64_t mat_rpc = is_mat ? (plan.ns_b + a->matrix_height - 1) / a->matrix_height : 1;
   const int64_t mat_cpc = is_mat ? (plan.ns_a + a->matrix_width - 1) / a->matrix_width : 1;
@@ -1065,8 +1067,10 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
   // Kernel choice: FP64 form, or the mixed band kernel (FP32 filter; for
   // 1NN_INDEX its candidates are verified, for SUM_THRESH the filter
   // threshold is the sum threshold and every cell above it is accumulated).
-  // The k-best and matrix-summary types run the FP64 visit kernel.
-  // FP64 1NN joins of some size run the band kernel's exact form.
+  // DOUBLE joins but sums run the band kernel's exact form (windows up to
+  // kExactMaxWindow; lists by exact_list(), grids by their entries' span); the FP64
+  // kernel is left with sums, ULTRA and longer windows, the visit kernels with
+  // ULTRA and what neither form of the band kernel takes.
   enum { K_FP64, K_MIXED, K_VISIT, K_EXACT } kind =
       visit ? K_VISIT : mixed ? K_MIXED : exact ? K_EXACT : K_FP64;
   const bool band = kind == K_MIXED || kind == K_EXACT;  // the FP32 band kernel's geometry
@@ -2027,9 +2031,11 @@ noalloc_prefix_kernel(JoinParams P, int64_t K, int W, int64_t* __restrict__ pref
   if (g < P.total_bands) prefix[g + 1] = part[g];
 }
 
-// The FP64 join of run_device() on the static scratch: the same kernels,
-// launch shapes and segment length, so the results equal
-// scamp_gb300_join_dev's.  Ordered on `st`; nothing is synchronised.
+// The plain FP64 join of run_device() on the static scratch: the same kernels,
+// launch shapes and segment length.  scamp_gb300_join_dev runs DOUBLE 1NN joins
+// in the exact form; both report FP64 re-evaluated correlations, so the results
+// are equal but for partners that tie within the recurrence's rounding.  Ordered
+// on `st`; nothing is synchronised.
 int run_device_noalloc(const NoAllocDevice& dv, const scamp_c_args* a, scamp_c_result* res,
                        cudaStream_t st, std::string* msg) {
   const int64_t na = static_cast<int64_t>(a->len_a);

@@ -1,8 +1,8 @@
 // join_mixed_1nn.cu -- the mixed-precision band kernel: FP32 filter over an
 // FP32 recurrence, exact path for the blocks it flags.  One body:
-// 1NN_INDEX mixed and double (each with a per-cell and a per-step-bound
-// filter), SUM_THRESH, APPROX_ALL_NEIGHBORS (k-best lists) and
-// MATRIX_SUMMARY.
+// 1NN_INDEX and SUM_THRESH in the mixed form (each with a per-cell and a
+// per-step-bound filter), APPROX_ALL_NEIGHBORS (k-best lists) and MATRIX_SUMMARY,
+// and the exact form of all but sums for DOUBLE joins (per-cell filter).
 //
 // Work decomposition as in join_fp64.cu (persistent kernel over a device
 // queue of units = band of kBand diagonals x two row segments of seg_len

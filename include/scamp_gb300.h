@@ -217,7 +217,7 @@ int scamp_gb300_join_batch(const scamp_c_args *args, scamp_c_result *res, int co
 int scamp_gb300_tune_batch(const scamp_c_args *args, int count, int retune, int64_t *segment,
                            char *errbuf, size_t errlen);
 
-/* The FP64 form of scamp_gb300_join_dev without any allocation: every
+/* scamp_gb300_join_dev on the plain FP64 kernels, without any allocation: every
  * intermediate buffer lives in one static device array of the library
  * (about 8.6 MB per device), so the join calls no allocator.  For callers
  * that must not allocate device memory at join time (a host that gives all
