@@ -412,7 +412,8 @@ struct Workspace {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t evk0 = nullptr, evk1 = nullptr;  // around the join kernels
   cudaEvent_t evkv = nullptr;                   // before the verification kernel
-  int fp64_occ = 1, visit_occ = 1;  // resident CTAs per SM of the FP64 and visit kernels
+  // resident CTAs per SM of the FP64 kernel and the visit kernels (lists, grid)
+  int fp64_occ = 1, visit_occ[2] = {1, 1};
   bool timed_kernel = false;
   bool timed_verify = false;
   // the mixed form's largest trusted drift margin (work counter 4) is the
@@ -1446,7 +1447,7 @@ int run_device(Workspace& ws, const scamp_c_args* a, scamp_c_result* res,
       if (is_1nn)
         join_fp64_kernel<<<static_cast<unsigned>(ws.sms * ws.fp64_occ), fp64_threads(), 0, st>>>(F);
       else
-        visit_fn<<<static_cast<unsigned>(ws.sms * ws.visit_occ), visit_threads(), 0, st>>>(
+        visit_fn<<<static_cast<unsigned>(ws.sms * ws.visit_occ[is_mat]), visit_threads(), 0, st>>>(
             F, visit_args());
       verify_exact_kernel<<<static_cast<unsigned>(ws.sms * 8), 256, 0, st>>>(F);
       launches += 2;
@@ -1638,9 +1639,11 @@ int init_workspace(int device, Workspace** out, std::string* msg) {
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &ws.fp64_occ, reinterpret_cast<const void*>(join_fp64_kernel), fp64_threads(), 0));
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &ws.visit_occ, reinterpret_cast<const void*>(join_visit_kernel), visit_threads(), 0));
+        &ws.visit_occ[0], reinterpret_cast<const void*>(join_visit_kernel), visit_threads(), 0));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &ws.visit_occ[1], reinterpret_cast<const void*>(join_visit_mat_kernel), visit_threads(), 0));
     ws.fp64_occ = std::max(ws.fp64_occ, 1);
-    ws.visit_occ = std::max(ws.visit_occ, 1);
+    for (int& occ : ws.visit_occ) occ = std::max(occ, 1);
     ws.device = device;
   }
   *out = &ws;
